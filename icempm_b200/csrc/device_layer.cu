@@ -70,7 +70,8 @@ struct Binning {
     int *key = nullptr, *count = nullptr, *cell_start = nullptr, *cursor = nullptr, *perm = nullptr;
     int *chunk = nullptr, *tile_start = nullptr, *pid = nullptr;
     int *group_slots = nullptr, *group_base = nullptr, *gchunk = nullptr;
-    int *lane_cell = nullptr, *cell_lane = nullptr;  // lane order of the cells of each tile
+    uint32_t *lane_cell = nullptr;  // lane order of the cells of each tile (TileRun::lane_cell)
+    int *cell_lane = nullptr;       // and the lane of each cell
     int *nbusy = nullptr;                            // tiles holding particles (1 int)
     size_t cap_pts = 0, cap_cells = 0, cap_tiles = 0, cap_slots = 0;
 };
@@ -95,6 +96,11 @@ struct Fused {
 };
 
 }  // namespace
+
+// the last answer of pair_threads and what it was for
+struct PairThreads {
+    int threads = 0, nbusy = -1, cells = 0, answer = 0;
+};
 
 struct icm_ctx {
     int device = 0;
@@ -144,6 +150,7 @@ struct icm_ctx {
     int nslots = 0;
     int *h_ns = nullptr;  // pinned: the slot count and busy tiles a re-binning reads back
     int nbusy = 0;        // tiles holding particles in the current binning
+    PairThreads wide;     // threads of the fused launches (pair_threads)
     // TMA descriptors of the three grid buffers (device copy) and what they
     // were encoded for
     CUtensorMap *d_tmap = nullptr;
@@ -509,17 +516,65 @@ static void opted_in(size_t *opted, int device, size_t dyn)
     if (device >= 0 && device < kMaxDevices) opted[device] = dyn;
 }
 
+// more warps than a tile has groups of 32 cells, and as many for each
+static bool pair_wide(int cells, int threads) { return threads > cells && threads % cells == 0; }
+
+// the pair loop's static shared memory (the lists of at most 16 groups), and room for the rest
+constexpr size_t kPairStaticBytes = 16 * (384 + 8) + 1024;
+
+// Threads per CTA of the pair loop: the block size asked for, doubled up to
+// 512 while the CTAs of the tiles with particles would all be resident at
+// once. A launch of few tiles lasts as long as its slowest tile, whose
+// warps' groups then run side by side (and, with more warps than groups, the
+// pairs of rounds of a group). memo keeps the last answer of a caller.
+static int pair_threads(int device, int cells, const void *kernel, const void *wide, size_t (*dyn_bytes)(int),
+                        int threads, int nbusy, PairThreads &memo, int &out)
+{
+    out = threads;
+    if (memo.threads == threads && memo.nbusy == nbusy && memo.cells == cells) {
+        out = memo.answer;
+        return ICM_OK;
+    }
+    int sms = 0, most = 0;
+    ICM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    ICM_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    // a power of two of warps shares the groups of every tile evenly
+    while ((out & (out - 1)) == 0 && out * 2 <= 32 * kPairMaxWarps && out * 2 <= cells * kPairWidest) {
+        const size_t dyn = dyn_bytes(2 * out / 32);
+        int per_sm = 0;
+        if (dyn + kPairStaticBytes > (size_t)most) break;
+        const void *k = pair_wide(cells, 2 * out) ? wide : kernel;
+        // (all there is: a smaller value would take back what a launch opted in to)
+        ICM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)kPairStaticBytes));
+        ICM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 2 * out, dyn));
+        if (nbusy > per_sm * sms) break;
+        out *= 2;
+    }
+    memo.threads = threads;
+    memo.nbusy = nbusy;
+    memo.cells = cells;
+    memo.answer = out;
+    return ICM_OK;
+}
+
 // Dynamic shared memory of the per-warp accumulation regions; above 48 KB
 // the kernel has to opt in once.
 template <class Pol, int TX, int TY, int MODE>
 static int launch_one(icm_ctx *c, int ntiles, const icy_SimParams &P, const typename Pol::Consts &K,
                       const typename Pol::Parts &A, const TileRun &R)
 {
-    constexpr int RN = (TX + 4) * (TY + 4);
-    const int nwarps = c->threads / 32;
-    if (TX * TY > 32 * kMaxGroupsPerWarp * nwarps || nwarps > kMaxWarps)
+    int threads = c->threads;
+    if (TX * TY > 32 * kMaxGroupsPerWarp * (threads / 32) || threads / 32 > kMaxWarps)
         return icm::fail(ICM_ERR_ARG, "tile too large for the block size (need threads >= TX*TY/4)");
-    const size_t dyn = tile_dyn_bytes<Pol, MODE>(RN, nwarps);
+    if constexpr (kPairLaunch<Pol, MODE>) {
+        const int rc = pair_threads(c->device, TX * TY, (const void *)k_tile_substep<Pol, TX, TY, kModeFull>,
+                                    (const void *)k_tile_substep<Pol, TX, TY, kModeFullWide>,
+                                    launch_dyn_bytes<Pol, TX, TY, MODE>, c->threads, c->nbusy, c->wide, threads);
+        if (rc) return rc;
+        if constexpr (MODE == kModeFull)
+            if (pair_wide(TX * TY, threads)) return launch_one<Pol, TX, TY, kModeFullWide>(c, ntiles, P, K, A, R);
+    }
+    const size_t dyn = launch_dyn_bytes<Pol, TX, TY, MODE>(threads / 32);
     static size_t opted[kMaxDevices] = {};  // static + dynamic shared memory above 48 KB needs the opt-in
     if (need_opt_in(opted, c->device, dyn)) {
         ICM_CUDA(cudaFuncSetAttribute(k_tile_substep<Pol, TX, TY, MODE>,
@@ -531,7 +586,7 @@ static int launch_one(icm_ctx *c, int ntiles, const icy_SimParams &P, const type
     // until it has completed
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ntiles);
-    cfg.blockDim = dim3(c->threads);
+    cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = dyn;
     cfg.stream = c->stream;
     cudaLaunchAttribute at[1];
@@ -839,7 +894,6 @@ static int run_fused(icm_ctx *c, icy_SimParams *p, int n)
     R.bins = c->d_bins;
     R.err = c->d_err;
     R.fp64_redo = c->d_redo;
-    R.cell_start = c->bin.cell_start;
     R.lane_cell = c->bin.lane_cell;
     R.group_base = c->bin.group_base;
     R.strays = c->d_strays;
@@ -890,7 +944,7 @@ static int run_fused(icm_ctx *c, icy_SimParams *p, int n)
         return r;
     };
     // prologue: P2G of the current state into G[0]
-    R.bufA = 0; R.bufB = 0; R.bufC = 0;
+    R.set_buffers(0, 0, 0);
     R.force_slot = nullptr;
     R.record_pq = 0;
     R.ind_x = p->indenter_x;
@@ -901,9 +955,7 @@ static int run_fused(icm_ctx *c, icy_SimParams *p, int n)
         t += p->InitialTimeStep;
         p->indenter_x = p->indenter_x_initial + t * p->IndVelocity;
         const int sidx = k - 1;
-        R.bufA = sidx % 3;
-        R.bufB = (sidx + 1) % 3;
-        R.bufC = (sidx + 2) % 3;
+        R.set_buffers(sidx % 3, (sidx + 1) % 3, (sidx + 2) % 3);
         R.ind_x = p->indenter_x;
         R.force_slot = c->d_hist + 2 * (size_t)sidx;
         R.record_pq = ((p->SimulationStep + k) % p->UpdateEveryNthStep == 0) ? 1 : 0;
@@ -1342,6 +1394,8 @@ struct icm_ensemble {
     int *d_tile_case = nullptr, *d_tile_local = nullptr, *d_nactive = nullptr, *d_seg_base = nullptr;
     size_t tiles_cap = 0;
     int nactive = 0;
+    int nbusy = 0;     // launch list entries of tiles with particles
+    PairThreads wide;  // threads of the launches (pair_threads)
     double *d_ind_x = nullptr;
     size_t ind_x_cap = 0;
     uint8_t *d_active = nullptr;  // every case's tile mask, concatenated
@@ -1349,7 +1403,7 @@ struct icm_ensemble {
     std::vector<size_t> active_off;
     struct Seg {
         cudaGraphExec_t exec;
-        int len, grid;
+        int len, grid, threads;
     };
     std::vector<Seg> graphs_by_len;  // captured segments (at most kEnsGraphs lengths)
     std::vector<cudaEvent_t> events;  // one per case, plus one for the ensemble stream
@@ -1380,10 +1434,17 @@ int ens_launch_one(icm_ensemble *e, int grid, const void *d_cases, const EnsLaun
     // the first launch of a segment, the prologue and the final launch follow
     // k_set_int or the descriptor upload, whose writes the kernel reads before
     // its dependency wait: they are ordinary stream-ordered launches
-    const bool pdl = MODE == kModeFull && L.j > 0;
-    constexpr int RN = (TX + 4) * (TY + 4);
-    const int nwarps = e->threads / 32;
-    const size_t dyn = tile_dyn_bytes<Pol, MODE>(RN, nwarps);
+    const bool pdl = (MODE == kModeFull || MODE == kModeFullWide) && L.j > 0;
+    int threads = e->threads;
+    if constexpr (kPairLaunch<Pol, MODE>) {
+        const int rc = pair_threads(e->device, TX * TY, (const void *)k_tile_substep_ens<Pol, TX, TY, kModeFull>,
+                                    (const void *)k_tile_substep_ens<Pol, TX, TY, kModeFullWide>,
+                                    launch_dyn_bytes<Pol, TX, TY, MODE>, e->threads, e->nbusy, e->wide, threads);
+        if (rc) return rc;
+        if constexpr (MODE == kModeFull)
+            if (pair_wide(TX * TY, threads)) return ens_launch_one<Pol, TX, TY, kModeFullWide>(e, grid, d_cases, L);
+    }
+    const size_t dyn = launch_dyn_bytes<Pol, TX, TY, MODE>(threads / 32);
     static size_t opted[kMaxDevices] = {};
     if (need_opt_in(opted, e->device, dyn)) {
         ICM_CUDA(cudaFuncSetAttribute(k_tile_substep_ens<Pol, TX, TY, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1395,7 +1456,7 @@ int ens_launch_one(icm_ensemble *e, int grid, const void *d_cases, const EnsLaun
     // (inside a captured segment this becomes a programmatic graph edge)
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(e->threads);
+    cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = dyn;
     cfg.stream = e->stream;
     cudaLaunchAttribute at[1];
@@ -1496,7 +1557,6 @@ int ens_upload_cases(icm_ensemble *e, const std::vector<icy_SimParams> &P, icy_S
         d.R.bins = c->d_bins;
         d.R.err = c->d_err;
         d.R.fp64_redo = c->d_redo;
-        d.R.cell_start = c->bin.cell_start;
         d.R.lane_cell = c->bin.lane_cell;
         d.R.group_base = c->bin.group_base;
         d.R.strays = c->d_strays;
@@ -1623,6 +1683,7 @@ int ens_active_tiles(icm_ensemble *e, const std::vector<icy_SimParams> &P)
         tc[k] = items[k].c;
         tl[k] = items[k].t;
     }
+    e->nbusy = (int)nbusy;
     const size_t m = items.size();
     int rc;
     if (m > e->tiles_cap) {
@@ -1675,8 +1736,12 @@ int ens_check(icm_ensemble *e)
 // return, so a graph captured for a longer list stays valid).
 int ens_segment_graph(icm_ensemble *e, int len, cudaGraphExec_t &out)
 {
+    // sets the kernel's shared-memory attribute and block size outside the
+    // capture (grid 0 launches nothing)
+    int rc0 = ens_launch(e, kModeFull, 0, 0);
+    if (rc0) return rc0;
     for (auto &g : e->graphs_by_len)
-        if (g.len == len && g.grid >= e->nactive) {
+        if (g.len == len && g.grid >= e->nactive && g.threads == e->wide.answer) {
             out = g.exec;
             return ICM_OK;
         }
@@ -1686,9 +1751,6 @@ int ens_segment_graph(icm_ensemble *e, int len, cudaGraphExec_t &out)
             e->graphs_by_len.erase(e->graphs_by_len.begin() + i);
             break;
         }
-    // set the kernel's shared-memory attribute outside the capture (grid 0 launches nothing)
-    int rc0 = ens_launch(e, kModeFull, 0, 0);
-    if (rc0) return rc0;
     cudaGraph_t g = nullptr;
     ICM_CUDA(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
     int rc = ICM_OK;
@@ -1703,7 +1765,7 @@ int ens_segment_graph(icm_ensemble *e, int len, cudaGraphExec_t &out)
     const cudaError_t ie = cudaGraphInstantiate(&ex, g, 0);
     cudaGraphDestroy(g);
     if (ie != cudaSuccess) return icm::fail(ICM_ERR_CUDA, std::string("ensemble graph: ") + cudaGetErrorString(ie));
-    e->graphs_by_len.push_back({ex, len, e->nactive});
+    e->graphs_by_len.push_back({ex, len, e->nactive, e->wide.answer});
     out = ex;
     return ICM_OK;
 }

@@ -54,7 +54,9 @@
 
 namespace icm {
 
-enum { kModeP2GOnly = 0, kModeFull = 1, kModeFinal = 2 };
+// kModeFullWide: a full substep of the pair loop with more warps than a tile
+// has groups
+enum { kModeP2GOnly = 0, kModeFull = 1, kModeFinal = 2, kModeFullWide = 3 };
 constexpr int kMaxBins = 256;
 // a CTA has at most 8 warps and each warp at most 4 groups of 32 cells, so
 // a tile of TX*TY cells needs at least TX*TY/128 warps
@@ -220,20 +222,33 @@ struct CellSumsComp {
     }
 };
 
+// a word of TileRun::lane_cell: the particle count in the low bits (65,536
+// stands for every count above 65,535)
+constexpr int kLaneCountBits = 17, kLaneCountMax = 65536;
+constexpr uint32_t kLaneCountMask = (1u << kLaneCountBits) - 1u;
+
 struct TileRun {
     int ntx, nty;
     const int *tile_start;   // ntiles + 1
     uint8_t *dirty[3];       // ntiles flags per buffer
     void *grid[3];
     int bufA, bufB, bufC;    // read / scatter / zero
+    void *gA, *gB, *gC;      // grid[bufA] .. (set_buffers)
+    uint8_t *dA, *dB, *dC;   // dirty[bufA] ..
+    __host__ __device__ void set_buffers(int a, int b, int c)
+    {
+        bufA = a; bufB = b; bufC = c;
+        gA = grid[a]; gB = grid[b]; gC = grid[c];
+        dA = dirty[a]; dB = dirty[b]; dC = dirty[c];
+    }
     double ind_x, ind_y;
     double *bins;            // 2*n_indenter_subdivisions, accumulated
     double *force_slot;      // 2 doubles: this substep's summed reaction
     int *err;
     int record_pq;
     unsigned long long *fp64_redo;
-    const int *cell_start;          // binning: cell key k holds cell_start[k+1] - cell_start[k] particles
-    const int *lane_cell;           // the cell key at each lane (tile by tile, fullest cells first)
+    const uint32_t *lane_cell;      // the cell at each lane (tile by tile, fullest cells first): its place in
+                                    // the tile << kLaneCountBits | its particle count (at most kLaneCountMax)
     const int *group_base;          // first slot of each group of 32 consecutive lanes
     unsigned long long *strays;     // particles that left their binned cell (count)
     // tile scheduling: CTA i runs tile order[i] (tile i when null); a full
@@ -277,17 +292,23 @@ constexpr int kTmaPolls = 1 << 22;
 // (A descriptor in global memory must have been fenced for the tensor-map
 // proxy by the issuing thread before this; one in kernel parameters needs
 // nothing.)
+__device__ __forceinline__ void tma_region_load(const CUtensorMap *map, void *dst, int rx0, int ry0, uint32_t bytes,
+                                                uint64_t *bar)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc05::smem_u32(bar)), "r"(bytes)
+                 : "memory");
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
+                 "[%4];" ::"r"(tc05::smem_u32(dst)),
+                 "l"(map), "r"(4 * rx0), "r"(ry0), "r"(tc05::smem_u32(bar))
+                 : "memory");
+}
+
 __device__ __forceinline__ void tma_region_issue(const CUtensorMap *map, void *dst, int rx0, int ry0, uint32_t bytes,
                                                  uint64_t *bar)
 {
     if (threadIdx.x == 0) {
         tc05::mbar_init(bar, 1);
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc05::smem_u32(bar)), "r"(bytes)
-                     : "memory");
-        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
-                     "[%4];" ::"r"(tc05::smem_u32(dst)),
-                     "l"(map), "r"(4 * rx0), "r"(ry0), "r"(tc05::smem_u32(bar))
-                     : "memory");
+        tma_region_load(map, dst, rx0, ry0, bytes, bar);
     }
 }
 
@@ -337,6 +358,7 @@ struct Pol64 {
     static constexpr bool kHarvest = false;  // Consts has no harvest fields
     // registers per thread: three 128-thread CTAs per SM
     static constexpr int kMaxRegs = 168;
+    static constexpr bool kPairs = false;  // the pair loop of k_pair32.cuh
     // staging rounds per warp (the particle state of a round is copied into
     // shared memory kStages - 1 rounds ahead); three would cost the FP64
     // form its third CTA per SM
@@ -376,6 +398,21 @@ struct Pol64 {
         return s;
     }
 
+    // six terms of a particle's P2G in the lane's place of a staged round
+    static __device__ __forceinline__ void stash(Stage &S, int lane, double c0, double c1, double S00, double S01,
+                                                 double S10, double S11)
+    {
+        S.F[lane] = make_double4(c0, c1, S00, S01);
+        S.pos[lane] = make_double2(S10, S11);
+    }
+    static __device__ __forceinline__ void unstash(const Stage &S, int lane, double &c0, double &c1, double &S00,
+                                                   double &S01, double &S10, double &S11)
+    {
+        const double4 a = S.F[lane];
+        const double2 b = S.pos[lane];
+        c0 = a.x; c1 = a.y; S00 = a.z; S01 = a.w;
+        S10 = b.x; S11 = b.y;
+    }
     static __device__ __forceinline__ void init_tables(Tables &, const Consts &, int, int) {}
     static __device__ __forceinline__ Sten stencil(const icy_SimParams &P, const Consts &, const St &s)
     {
@@ -469,6 +506,8 @@ struct Pol32 {
     static constexpr bool kHarvest = true;
     // registers per thread: four 128-thread CTAs per SM
     static constexpr int kMaxRegs = 128;
+    // full substeps walk the particles of a cell in pairs (k_pair32.cuh)
+    static constexpr bool kPairs = true;
     // staging rounds per warp (the particle state of a round is copied into
     // shared memory kStages - 1 rounds ahead)
     static constexpr int kStages = 2;
@@ -492,6 +531,8 @@ struct Pol32 {
     struct Sten { int bx, by; float fx, fy, wx[3], wy[3]; };
     // one round of a warp (32 particles) staged in shared memory
     struct Stage { float4 H[32]; float4 X[32]; float Jp[32]; };
+    // one iteration of the pair loop: two rounds
+    struct PairStage { float4 H[2][32]; float4 X[2][32]; float Jp[2][32]; };
 
     static __device__ __forceinline__ void prefetch(const Parts &A, int p, Stage &S, int lane)
     {
@@ -515,6 +556,20 @@ struct Pol32 {
         return unpack(S.X[lane], S.H[lane], S.Jp[lane]);
     }
 
+    // six terms of a particle's P2G in the lane's place of a staged round
+    static __device__ __forceinline__ void stash(Stage &S, int lane, float c0, float c1, float S00, float S01, float S10,
+                                                 float S11)
+    {
+        S.H[lane] = make_float4(c0, c1, S00, S01);
+        S.X[lane] = make_float4(S10, S11, 0.f, 0.f);
+    }
+    static __device__ __forceinline__ void unstash(const Stage &S, int lane, float &c0, float &c1, float &S00, float &S01,
+                                                   float &S10, float &S11)
+    {
+        const float4 a = S.H[lane], b = S.X[lane];
+        c0 = a.x; c1 = a.y; S00 = a.z; S01 = a.w;
+        S10 = b.x; S11 = b.y;
+    }
     static __device__ __forceinline__ void init_tables(Tables &T, const Consts &K, int tid, int nthr)
     {
         grain_tables32_init(T, K, tid, nthr);
@@ -634,7 +689,8 @@ struct Pol32 {
     {
         if (meta32_crushed(s.meta) && k.harvest) harvest_state(k, s.H, s.Jp, s.meta);
     }
-    static __device__ __forceinline__ Tau<float> advance(const icy_SimParams &P, const Consts &k, const Tables &T,
+    template <class Strengths>
+    static __device__ __forceinline__ Tau<float> advance(const icy_SimParams &P, const Consts &k, const Strengths &T,
                                                          St &s, float v0, float v1, const float B[4], float &p_tr,
                                                          float &q_tr, int &redo)
     {
@@ -751,6 +807,7 @@ static __device__ __noinline__ SurrogateOut surrogate_finish(const icy_SimParams
 // Jp_inv < 1, a closed form with nothing to learn), the exact map runs.
 struct Pol32S : Pol32 {
     static constexpr bool kSurrogate = true;
+    static constexpr bool kPairs = false;
     // two staging rounds: a third would not leave room for four CTAs per SM
     // next to the network's rows
     static constexpr int kStages = 2;
@@ -843,6 +900,7 @@ struct Pol32S : Pol32 {
 // registers beyond the FP32 form's 128, so this form runs three 128-thread
 // CTAs per SM.
 struct Pol32C : Pol32 {
+    static constexpr bool kPairs = false;
     using Sums = CellSumsComp;
     static constexpr int kMaxRegs = 168;
 };
@@ -1010,6 +1068,43 @@ __device__ __forceinline__ int group_of(int j, int warp, int nwarps, int part)
     return part == 0 ? m : 2 * m + (part - 1);
 }
 
+// The same by the whole warp, for the particle at slot p that lane l of a
+// round put aside (its terms c and S stashed in the round's staging space,
+// its new position in the particle arrays): lane q < 9 adds the contribution
+// to node (q / 3, q % 3), inside the region with plain additions. A float
+// addition to shared memory is a compare-and-swap loop; 27 of them by the
+// particle's own lane took several thousand instructions.
+template <class Pol, int TX, int TY>
+__device__ __forceinline__ int stray_scatter(const icy_SimParams &P, const typename Pol::Consts &K,
+                                             const typename Pol::Parts &A, const TileRun &R, const int p,
+                                             const typename Pol::Stage &S, const int l, typename Pol::Acc *wacc,
+                                             const int rx0, const int ry0, const typename Pol::real m)
+{
+    using real = typename Pol::real;
+    constexpr int RX = TX + 4, RY = TY + 4;
+    const int lane = threadIdx.x & 31, i = lane / 3, j = lane % 3;
+    int bad = 0;
+    if (lane < 9) {
+        const typename Pol::Sten st = Pol::stencil(P, K, Pol::load(A, p));
+        real c0, c1, S00, S01, S10, S11;
+        Pol::unstash(S, l, c0, c1, S00, S01, S10, S11);
+        const real W = (i == 0 ? st.wx[0] : i == 1 ? st.wx[1] : st.wx[2]) * (j == 0 ? st.wy[0] : j == 1 ? st.wy[1] : st.wy[2]);
+        const real mm = W * m, mx = W * (c0 + S00 * (real)i + S01 * (real)j), my = W * (c1 + S10 * (real)i + S11 * (real)j);
+        const int lx = st.bx - rx0, ly = st.by - ry0, gx = st.bx + i, gy = st.by + j;
+        if (lx >= 0 && ly >= 0 && lx + 2 < RX && ly + 2 < RY && st.bx >= 0 && st.by >= 0 && st.bx + 2 < P.GridX &&
+            st.by + 2 < P.GridY) {
+            acc_add(wacc[(ly + j) * RX + lx + i], mm, mx, my);
+        } else if (gx < 0 || gy < 0 || gx >= P.GridX || gy >= P.GridY) {
+            bad = 1;
+        } else {
+            node_add_global((typename Pol::Node *)R.gB, (size_t)gy * P.GridX + gx, mm, mx, my);
+            R.dB[(gy / TY) * R.ntx + gx / TX] = 1;
+        }
+    }
+    __syncwarp();
+    return bad;
+}
+
 // Whether a node of tile t's (TX+4) x (TY+4) region lies inside the
 // indenter's circle.
 template <int TX, int TY>
@@ -1049,8 +1144,7 @@ __host__ __device__ constexpr size_t tile_dyn_bytes(int RN, int nwarps)
 template <class Pol, int TX, int TY, int MODE>
 __device__ __forceinline__ void tile_body(const icy_SimParams &P, const typename Pol::Consts &K,
                                           const typename Pol::Parts &A, const TileRun &R, const int t,
-                                          const CUtensorMap *tmaps, const bool tmaps_in_global, const int part,
-                                          const bool pdl_wait)
+                                          const CUtensorMap *tmaps, const bool tmaps_in_global, const int part)
 {
     using real = typename Pol::real;
     using V2 = typename Pol::V2;
@@ -1078,8 +1172,8 @@ __device__ __forceinline__ void tile_body(const icy_SimParams &P, const typename
     // force bins and total of the tile's contact nodes, in the staging space
     double *s_bins = reinterpret_cast<double *>(s_dyn + tile_region_bytes<Pol, MODE>(RN, nthr >> 5));
     double *s_tot = s_bins + 2 * kMaxBins;
-    Node *gA = (Node *)R.grid[R.bufA];
-    Node *gB = (Node *)R.grid[R.bufB];
+    Node *gA = (Node *)R.gA;
+    Node *gB = (Node *)R.gB;
     const unsigned FULL = 0xffffffffu;
     const int lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
     constexpr int CELLS = TX * TY;
@@ -1096,13 +1190,13 @@ __device__ __forceinline__ void tile_body(const icy_SimParams &P, const typename
     int ng_w = 0;
     if (p1 > p0) {
         for (int g; (g = group_of(ng_w, warp, nwarps, part)) < NGT_; ng_w++) {
-            const int c = R.lane_cell[t * CELLS + g * 32 + lane];
-            int cnt = R.cell_start[c + 1] - R.cell_start[c];
+            const uint32_t lc = R.lane_cell[t * CELLS + g * 32 + lane];
+            int cnt = (int)(lc & kLaneCountMask);
             if (cnt > 0xffff) {  // beyond the count field: the cell's later particles are not advanced
                 atomicOr(R.err, kErrCellOverflow);
                 cnt = 0xffff;
             }
-            s_wcnt[warp][ng_w][lane] = ((uint32_t)(c - t * CELLS) << 16) | (uint32_t)cnt;
+            s_wcnt[warp][ng_w][lane] = ((lc >> kLaneCountBits) << 16) | (uint32_t)cnt;
             const int rounds = __reduce_max_sync(FULL, cnt);
             if (lane == 0) {
                 s_wrounds[warp][ng_w] = rounds;
@@ -1126,10 +1220,8 @@ __device__ __forceinline__ void tile_body(const icy_SimParams &P, const typename
     // launched as a programmatic dependent: wait until the previous kernel
     // of the stream has completed and its writes are visible, then let the
     // next one launch (its CTAs take free slots, set up, and wait here)
-    if (pdl_wait) {
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // the node region's copy into the (not yet used) accumulation regions,
     // issued right after the wait so that it lands while the tile zeroes
     // its next-but-one buffer
@@ -1139,17 +1231,17 @@ __device__ __forceinline__ void tile_body(const icy_SimParams &P, const typename
 
     // 1. zero this tile in the buffer the next substep will scatter into;
     //    the flag is cleared only after every thread has read it
-    const bool zero_c = (MODE == kModeFull) && part != 2 && R.dirty[R.bufC][t];
+    const bool zero_c = (MODE == kModeFull) && part != 2 && R.dC[t];
     if (zero_c) {
-        Node *gC = (Node *)R.grid[R.bufC];
+        Node *gC = (Node *)R.gC;
         for (int k = tid; k < TX * TY; k += nthr) {
             int gx = x0 + k % TX, gy = y0 + k / TX;
             if (gx < GX && gy < GY) node_zero(gC, (size_t)gy * GX + gx);
         }
         __syncthreads();
-        if (tid == 0) R.dirty[R.bufC][t] = 0;
+        if (tid == 0) R.dC[t] = 0;
     }
-    const bool has_mass = (MODE != kModeP2GOnly) && R.dirty[R.bufA][t];
+    const bool has_mass = (MODE != kModeP2GOnly) && R.dA[t];
     const int np = p1 - p0;
     if (np == 0 && !has_mass) return;
 
@@ -1304,6 +1396,7 @@ __device__ __forceinline__ void tile_body(const icy_SimParams &P, const typename
         // stray path, which raises the error word as v2_kernel_p2g does
         const bool cell_ok = cbx + 2 < GX && cby + 2 < GY;
         if (r == 0) sums.zero();
+        bool deferred = false, stray = false;
         // P2G of one (updated) particle: node (i, j) gets
         // W_ij (m, c + S_h (i, j)^T) with S = m Bp - dt Vp Dinv tau
         auto p2g = [&](const typename Pol::St &s, const real v0, const real v1, const real *B,
@@ -1315,11 +1408,9 @@ __device__ __forceinline__ void tile_body(const icy_SimParams &P, const typename
             const real c1 = v1 * m - (S10 * st.fx + S11 * st.fy);
             if (cell_ok && st.bx == cbx && st.by == cby) {
                 sums.add(st.wx, st.wy, m, c0, c1, S00, S01, S10, S11);
-            } else {
-                stray_count++;
-                bad |= stray_p2g<Pol, TX, TY>(wacc, rx0, ry0, GX, GY, gB, R.dirty[R.bufB], R.ntx, st.bx, st.by,
-                                              st.wx[0], st.wx[1], st.wx[2], st.wy[0], st.wy[1], st.wy[2], m, c0, c1,
-                                              S00, S01, S10, S11);
+            } else {  // scattered below; its terms wait in the staging space, already read
+                stray = true;
+                Pol::stash(stage[cur], lane, c0, c1, S00, S01, S10, S11);
             }
         };
         // the lane's cell sums into the warp's region: 9 read-modify-write
@@ -1336,7 +1427,6 @@ __device__ __forceinline__ void tile_body(const icy_SimParams &P, const typename
                     __syncwarp();
                 }
         };
-        bool deferred = false;
         if (r < cnt) {
             const int p = s_wgbase[warp][k] + 32 * r + lane;
             typename Pol::St s = Pol::load_staged(stage[cur], lane);
@@ -1492,6 +1582,18 @@ __device__ __forceinline__ void tile_body(const icy_SimParams &P, const typename
                 }
             }
         }
+        if (MODE != kModeFinal) {
+            unsigned out = __ballot_sync(FULL, stray);
+            if (out) {
+                __syncwarp();
+                stray_count += stray;
+                for (; out; out &= out - 1) {
+                    const int l = __ffs(out) - 1;
+                    bad |= stray_scatter<Pol, TX, TY>(P, K, A, R, s_wgbase[warp][k] + 32 * r + l, stage[cur], l, wacc, rx0,
+                                                      ry0, m);
+                }
+            }
+        }
         // last round of this group: its cells' sums go to the warp's region
         if (MODE != kModeFinal && nk != k) flush_cell_sums();
         k = nk;
@@ -1533,26 +1635,63 @@ __device__ __forceinline__ void tile_body(const icy_SimParams &P, const typename
     __syncthreads();
     if (tid < 9 && s_mark[tid]) {
         int ntx2 = tx + tid % 3 - 1, nty2 = ty + tid / 3 - 1;
-        if (ntx2 >= 0 && nty2 >= 0 && ntx2 < R.ntx && nty2 < R.nty) R.dirty[R.bufB][nty2 * R.ntx + ntx2] = 1;
+        if (ntx2 >= 0 && nty2 >= 0 && ntx2 < R.ntx && nty2 < R.nty) R.dB[nty2 * R.ntx + ntx2] = 1;
+    }
+}
+
+// What a tile without particles has to do in a substep: zero its nodes in
+// the next-but-one buffer (zero), and add the reaction of its own nodes (the
+// grid update's contact, gpu_implementation5.cu:245-271) to the force bins
+// with global FP64 atomics (contact).
+template <class Pol, int TX, int TY>
+__device__ __forceinline__ void empty_tile(const icy_SimParams &P, const typename Pol::Consts &K, const TileRun &R,
+                                           const int t, const bool zero, const bool contact)
+{
+    using Node = typename Pol::Node;
+    using real = typename Pol::real;
+    const int GX = P.GridX, GY = P.GridY, tid = threadIdx.x, nthr = blockDim.x;
+    const int x0 = (t % R.ntx) * TX, y0 = (t / R.ntx) * TY;
+    if (zero) {
+        Node *gC = (Node *)R.gC;
+        for (int k = tid; k < TX * TY; k += nthr) {
+            const int gx = x0 + k % TX, gy = y0 + k / TX;
+            if (gx < GX && gy < GY) node_zero(gC, (size_t)gy * GX + gx);
+        }
+    }
+    if (contact) {
+        const Node *gA = (const Node *)R.gA;
+        for (int k = tid; k < TX * TY; k += nthr) {
+            const int gx = x0 + k % TX, gy = y0 + k / TX;
+            if (gx >= GX || gy >= GY) continue;
+            real v0, v1;
+            double f0 = 0, f1 = 0;
+            int bin;
+            Pol::node_velocity(P, K, gA[(size_t)gy * GX + gx], gx, gy, R.ind_x, R.ind_y, v0, v1, f0, f1, bin, true);
+            if (bin >= 0) {
+                atomicAdd(&R.bins[2 * bin], f0);
+                atomicAdd(&R.bins[2 * bin + 1], f1);
+                if (R.force_slot) {
+                    atomicAdd(&R.force_slot[0], f0);
+                    atomicAdd(&R.force_slot[1], f1);
+                }
+            }
+        }
     }
 }
 
 // Tiles without particles, kEmptyPerCta of them per CTA (an empty group of
 // the launch order). Each one's nodes in the next-but-one buffer are zeroed
 // where its dirty flag says so, and a tile that holds mass and that the
-// indenter can reach adds the reaction of its own nodes (the grid update's
-// contact, gpu_implementation5.cu:245-271) to the force bins with global
-// FP64 atomics. The group's flags are read at once, after the wait for the
-// previous substep, so that the latency of the loads is paid once per CTA.
+// indenter can reach adds the reaction of its own nodes. The group's flags
+// are read at once, after the wait for the previous substep, so that the
+// latency of the loads is paid once per CTA.
 template <class Pol, int TX, int TY, int MODE>
 __device__ __forceinline__ void empty_group(const icy_SimParams &P, const typename Pol::Consts &K, const TileRun &R,
                                             const int grp)
 {
-    using Node = typename Pol::Node;
-    using real = typename Pol::real;
     __shared__ int s_et[kEmptyPerCta];
     __shared__ uint8_t s_ez[kEmptyPerCta], s_ec[kEmptyPerCta];
-    const int tid = threadIdx.x, nthr = blockDim.x;
+    const int tid = threadIdx.x;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (tid < kEmptyPerCta) {
@@ -1561,48 +1700,44 @@ __device__ __forceinline__ void empty_group(const icy_SimParams &P, const typena
         uint8_t z = 0, c = 0;
         if (i < R.nempty) {
             t = R.empties[i];
-            z = (MODE == kModeFull) ? R.dirty[R.bufC][t] : 0;
-            c = (R.dirty[R.bufA][t] && region_touches_indenter<TX, TY>(P, R, t)) ? 1 : 0;
+            z = (MODE == kModeFull || MODE == kModeFullWide) ? R.dC[t] : 0;
+            c = (R.dA[t] && region_touches_indenter<TX, TY>(P, R, t)) ? 1 : 0;
         }
         s_et[tid] = t;
         s_ez[tid] = z;
         s_ec[tid] = c;
     }
     __syncthreads();
-    const int GX = P.GridX, GY = P.GridY;
     for (int j = 0; j < kEmptyPerCta; j++) {
         const int t = s_et[j];
         if (t < 0) continue;
-        const int x0 = (t % R.ntx) * TX, y0 = (t / R.ntx) * TY;
-        if (s_ez[j]) {
-            Node *gC = (Node *)R.grid[R.bufC];
-            for (int k = tid; k < TX * TY; k += nthr) {
-                const int gx = x0 + k % TX, gy = y0 + k / TX;
-                if (gx < GX && gy < GY) node_zero(gC, (size_t)gy * GX + gx);
-            }
-        }
-        if (s_ec[j]) {
-            const Node *gA = (const Node *)R.grid[R.bufA];
-            for (int k = tid; k < TX * TY; k += nthr) {
-                const int gx = x0 + k % TX, gy = y0 + k / TX;
-                if (gx >= GX || gy >= GY) continue;
-                real v0, v1;
-                double f0 = 0, f1 = 0;
-                int bin;
-                Pol::node_velocity(P, K, gA[(size_t)gy * GX + gx], gx, gy, R.ind_x, R.ind_y, v0, v1, f0, f1, bin, true);
-                if (bin >= 0) {
-                    atomicAdd(&R.bins[2 * bin], f0);
-                    atomicAdd(&R.bins[2 * bin + 1], f1);
-                    if (R.force_slot) {
-                        atomicAdd(&R.force_slot[0], f0);
-                        atomicAdd(&R.force_slot[1], f1);
-                    }
-                }
-            }
-        }
+        empty_tile<Pol, TX, TY>(P, K, R, t, s_ez[j], s_ec[j]);
     }
     __syncthreads();  // every thread's zeroing is done before the flags clear
-    if (tid < kEmptyPerCta && s_et[tid] >= 0 && s_ez[tid]) R.dirty[R.bufC][s_et[tid]] = 0;
+    if (tid < kEmptyPerCta && s_et[tid] >= 0 && s_ez[tid]) R.dC[s_et[tid]] = 0;
+}
+
+}  // namespace icm
+
+#include "k_pair32.cuh"
+
+namespace icm {
+
+// the body and the dynamic shared memory of a launch: the pair form where
+// the policy has one
+template <class Pol, int MODE> constexpr bool kPairLaunch = Pol::kPairs && (MODE == kModeFull || MODE == kModeFullWide);
+template <class Pol, int TX, int TY, int MODE>
+__device__ __forceinline__ void substep_body(const icy_SimParams &P, const typename Pol::Consts &K,
+                                             const typename Pol::Parts &A, const TileRun &R, const int t,
+                                             const CUtensorMap *tmaps, const bool tmaps_in_global, const int part)
+{
+    if constexpr (kPairLaunch<Pol, MODE>) pair_tile_body<TX, TY, MODE == kModeFullWide>(P, K, A, R, t, tmaps, tmaps_in_global, part);
+    else tile_body<Pol, TX, TY, MODE>(P, K, A, R, t, tmaps, tmaps_in_global, part);
+}
+template <class Pol, int TX, int TY, int MODE> __host__ __device__ constexpr size_t launch_dyn_bytes(int nwarps)
+{
+    constexpr int RN = (TX + 4) * (TY + 4);
+    return kPairLaunch<Pol, MODE> ? pair_dyn_bytes(RN, nwarps) : tile_dyn_bytes<Pol, MODE>(RN, nwarps);
 }
 
 // One launch = one substep over all tiles, one CTA per tile. Tile costs are
@@ -1613,7 +1748,8 @@ __device__ __forceinline__ void empty_group(const icy_SimParams &P, const typena
 template <class Pol, int TX, int TY, int MODE>
 __global__ void __maxnreg__(Pol::kMaxRegs) k_tile_substep(const __grid_constant__ icy_SimParams P,
                                                       const __grid_constant__ typename Pol::Consts K,
-                                                      const typename Pol::Parts A, const __grid_constant__ TileRun R,
+                                                      const __grid_constant__ typename Pol::Parts A,
+                                                      const __grid_constant__ TileRun R,
                                                       const __grid_constant__ TmapSet T)
 {
     __shared__ long long s_clock;
@@ -1633,9 +1769,9 @@ __global__ void __maxnreg__(Pol::kMaxRegs) k_tile_substep(const __grid_constant_
     }
     const int t = code & kTileMask;
     const int part = (code & kSplitBit) ? ((code & kHalfBit) ? 2 : 1) : 0;
-    if (MODE == kModeFull && threadIdx.x == 0) s_clock = clock64();
-    tile_body<Pol, TX, TY, MODE>(P, K, A, R, t, R.tmap ? T.m : nullptr, false, part, true);
-    if (MODE == kModeFull && R.cost) {
+    if ((MODE == kModeFull || MODE == kModeFullWide) && threadIdx.x == 0) s_clock = clock64();
+    substep_body<Pol, TX, TY, MODE>(P, K, A, R, t, R.tmap ? T.m : nullptr, false, part);
+    if ((MODE == kModeFull || MODE == kModeFullWide) && R.cost) {
         __syncthreads();
         if (threadIdx.x == 0) {
             // cost[t] and cost[ntiles + t]: the tile's two halves (the second
@@ -1708,16 +1844,14 @@ __global__ void __maxnreg__(Pol::kMaxRegs) k_tile_substep_ens(const EnsCase<Pol>
     __syncthreads();
     if (threadIdx.x == 0) {
         if (MODE == kModeP2GOnly) {
-            sc.R.bufA = sc.R.bufB = sc.R.bufC = 0;
+            sc.R.set_buffers(0, 0, 0);
             sc.R.force_slot = nullptr;
             sc.R.record_pq = 0;
             sc.R.ind_x = sc.P.indenter_x;
             ens_gate_harvest(sc, 0, false);
         } else {
             const int sidx = *L.seg_base + L.j;
-            sc.R.bufA = sidx % 3;
-            sc.R.bufB = (sidx + 1) % 3;
-            sc.R.bufC = (sidx + 2) % 3;
+            sc.R.set_buffers(sidx % 3, (sidx + 1) % 3, (sidx + 2) % 3);
             sc.R.ind_x = sc.ind_x[sidx];
             sc.R.force_slot = sc.hist + 2 * (size_t)sidx;
             sc.R.record_pq = (sc.step0 + sidx + 1) % sc.every == 0 ? 1 : 0;
@@ -1726,8 +1860,8 @@ __global__ void __maxnreg__(Pol::kMaxRegs) k_tile_substep_ens(const EnsCase<Pol>
         }
     }
     __syncthreads();
-    tile_body<Pol, TX, TY, MODE>(sc.P, sc.K, sc.A, sc.R, t, sc.R.tmap, true, part, true);
-    if (MODE == kModeFull && sc.R.cost) {
+    substep_body<Pol, TX, TY, MODE>(sc.P, sc.K, sc.A, sc.R, t, sc.R.tmap, true, part);
+    if ((MODE == kModeFull || MODE == kModeFullWide) && sc.R.cost) {
         __syncthreads();
         if (threadIdx.x == 0) {
             const long long dc = clock64() - s_clock;
@@ -2041,9 +2175,9 @@ __global__ void k_bin_order(int ncells, const int *start, int *perm)
 
 // Lane order of the cells of each tile (one warp per tile, cells_per_tile a
 // multiple of 32 and at most kMaxTileCells): by particle count, fullest
-// first, ties by cell key. lane_cell[l] is the cell key at lane l and
-// cell_lane its inverse; both index the tile's own range of keys,
-// t * cells_per_tile + i. A group of 32 consecutive lanes then holds cells of
+// first, ties by cell key. lane_cell[l] is the cell at lane l with its count
+// (see TileRun) and cell_lane the lane of each cell key; both index the
+// tile's own range of keys, t * cells_per_tile + i. A group of 32 consecutive lanes then holds cells of
 // similar counts, so that few of its lanes idle through the rounds of its
 // fullest cell. The same pass writes what follows from the order:
 // group_slots (32 x the count of the group's first, fullest lane: its slots
@@ -2055,7 +2189,7 @@ __global__ void k_bin_order(int ncells, const int *start, int *perm)
 constexpr int kMaxTileCells = 512, kLaneOrderWarps = 4;
 
 __global__ void __launch_bounds__(32 * kLaneOrderWarps) k_lane_order(int ntiles, int cells_per_tile,
-                                                                    const int *cell_start, int *lane_cell,
+                                                                    const int *cell_start, uint32_t *lane_cell,
                                                                     int *cell_lane, int *group_slots,
                                                                     int *tile_start, int *nbusy)
 {
@@ -2074,7 +2208,7 @@ __global__ void __launch_bounds__(32 * kLaneOrderWarps) k_lane_order(int ntiles,
     if (last == first) {
         // no particles: every count is 0, and the order by key is the identity
         for (int i = lane; i < cells_per_tile; i += 32) {
-            lane_cell[base + i] = base + i;
+            lane_cell[base + i] = (uint32_t)i << kLaneCountBits;
             cell_lane[base + i] = base + i;
         }
         if (lane < rows) group_slots[(base >> 5) + lane] = 0;
@@ -2103,7 +2237,7 @@ __global__ void __launch_bounds__(32 * kLaneOrderWarps) k_lane_order(int ntiles,
             const unsigned b = __ballot_sync(FULL, mine);
             if (mine) {
                 const int l = pos + __popc(b & below), cell = 32 * r + lane;
-                lane_cell[base + l] = base + cell;
+                lane_cell[base + l] = ((uint32_t)cell << kLaneCountBits) | (uint32_t)min(v, kLaneCountMax);
                 cell_lane[base + cell] = base + l;
                 if ((l & 31) == 0) group_slots[(base + l) >> 5] = 32 * v;
             }

@@ -73,12 +73,27 @@ __device__ __forceinline__ void grain_tables32_init(GrainTables32 &T, const Cons
     }
 }
 
-// meta word of the FP32 form: residues in bits 0-5, 6-11, 12-16; crushed
-// flag in bits 24-31.
+// The same strengths computed where they are needed instead of looked up.
+struct GrainStrengths32 {
+    const Consts32 &k;
+    struct Pmax { const Consts32 &k; __device__ float operator[](uint32_t r) const { return k.ics * (1.0f + k.gv * 0.05f * (float)(-10 + ((int)r - 20))); } };
+    struct Pmin { const Consts32 &k; __device__ float operator[](uint32_t r) const { return -k.its * (1.0f + k.gv * 0.033f * (float)(-15 + ((int)r - 29))); } };
+    struct Qmax { const Consts32 &k; __device__ float operator[](uint32_t r) const { return k.iss * (1.0f + k.gv * 0.1f * (float)(-10 + ((int)r - 10))); } };
+    Pmax pmax;
+    Pmin pmin;
+    Qmax qmax;
+    __device__ explicit GrainStrengths32(const Consts32 &K) : k(K), pmax{K}, pmin{K}, qmax{K} {}
+};
+
+// meta word of the FP32 form: residues in bits 0-5, 6-11, 12-16; bit 17 set
+// when all three are those of a non-negative grain id; crushed flag in bits
+// 24-31.
+constexpr uint32_t kMetaNonNeg = 1u << 17, kMetaCrushed = 0xff000000u;
 __host__ __device__ __forceinline__ uint32_t grain_meta32(int grain, int crushed)
 {
     uint32_t r1 = (uint32_t)(grain % 21 + 20), r2 = (uint32_t)((grain + 3) % 30 + 29), r3 = (uint32_t)((grain + 4) % 11 + 10);
-    return r1 | (r2 << 6) | (r3 << 12) | ((uint32_t)crushed << 24);
+    return r1 | (r2 << 6) | (r3 << 12) | (r1 >= 20u && r2 >= 29u && r3 >= 10u ? kMetaNonNeg : 0u) |
+           ((uint32_t)crushed << 24);
 }
 __device__ __forceinline__ int meta32_crushed(uint32_t m) { return (int)(m >> 24); }
 
@@ -133,7 +148,7 @@ __device__ __forceinline__ float approx_sqrt(float x) { return x > 0.0f ? x * rs
 // relative margin of the surface, where the FP32 decision is not trusted.
 constexpr float kSurfaceMargin = 1e-3f;
 
-__device__ __forceinline__ int failure_side32(const GrainTables32 &T, uint32_t meta, float p_pa, float q_pa)
+template <class Strengths> __device__ __forceinline__ int failure_side32(const Strengths &T, uint32_t meta, float p_pa, float q_pa)
 {
     float pmax = T.pmax[meta & 63u];
     float pmin = T.pmin[(meta >> 6) & 63u];
@@ -251,7 +266,8 @@ static __device__ __noinline__ Crushed32 crushed32(const Consts32 &k, const M2f 
 // or outside its failure surface or within kSurfaceMargin of it, for a
 // crushed one near a discontinuity of the map, and for det F <= 0.25.
 // jpm1 = Jp_inv - 1.
-__device__ __forceinline__ int constitutive32(const Consts32 &k, const GrainTables32 &T, M2f &H, float &jpm1,
+template <class Strengths>
+__device__ __forceinline__ int constitutive32(const Consts32 &k, const Strengths &T, M2f &H, float &jpm1,
                                               uint32_t meta, float &p_tr, float &q_tr, Tau32 &tau)
 {
     Inv32 v = invariants32(H, k.mu, k.kappa);
@@ -268,8 +284,7 @@ __device__ __forceinline__ int constitutive32(const Consts32 &k, const GrainTabl
         return kC32_OK;
     }
     float q = 2.0f * v.s1 * approx_sqrt(v.hd * v.hd + v.b01 * v.b01);
-    // residues at or above their offsets: the grain id is not negative
-    const bool grain_nonneg = (meta & 63u) >= 20u && ((meta >> 6) & 63u) >= 29u && ((meta >> 12) & 31u) >= 10u;
+    const bool grain_nonneg = (meta & kMetaNonNeg) != 0u;
     const float pm = p * 1e-6f, qm = q * 1e-6f;
     const bool clearly_inside = grain_nonneg && pm > k.inside_plo && pm < k.inside_phi && qm * qm < k.inside_q2;
     if (!clearly_inside && failure_side32(T, meta, p, q) != 0) return kC32_NEEDS_FP64;
