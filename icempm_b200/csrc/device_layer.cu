@@ -117,6 +117,7 @@ struct icm_ctx {
     icy_SimParams prms{};
     size_t cap_pts = 0, cap_nodes = 0, pts_pitch = 0, grid_pitch = 0;
     double *d_pts = nullptr, *d_grid = nullptr, *d_bins = nullptr;
+    double *d_grid2 = nullptr;  // step-wise form: the grid of every other substep
     int *d_err = nullptr;
     double *d_hist = nullptr;
     size_t hist_cap = 0;
@@ -977,33 +978,63 @@ static int run_fused(icm_ctx *c, icy_SimParams *p, int n)
     return ICM_OK;
 }
 
+// A launch on the context's stream as a programmatic dependent of the
+// kernel before it (the step-wise kernels wait for it themselves).
+template <class... KArgs, class... Args>
+static cudaError_t launch_dependent(cudaStream_t s, void (*kernel)(KArgs...), int blocks, int threads, Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 static int run_stepwise(icm_ctx *c, icy_SimParams *p, int n)
 {
     int rc = ensure_ref(c);
     if (rc) return rc;
     if ((rc = ensure_hist(c, n))) return rc;
     cudaStream_t s = c->stream;
+    const size_t grid_bytes = sizeof(double) * c->grid_pitch * ICM_N_GRID_ARRAYS;
+    if (!c->d_grid2) {  // the grids of two successive substeps
+        if ((rc = dalloc(&c->d_grid2, c->grid_pitch * ICM_N_GRID_ARRAYS))) return rc;
+        ICM_CUDA(cudaMemsetAsync(c->d_grid2, 0, grid_bytes, s));
+    }
     ICM_CUDA(cudaMemsetAsync(c->d_hist, 0, sizeof(double) * 2 * (size_t)n, s));
+    // the last substep leaves its grid in d_grid, where callers can read it
+    double *grids[2] = {c->d_grid, c->d_grid2};
+    ICM_CUDA(cudaMemsetAsync(grids[(n - 1) & 1], 0, grid_bytes, s));
+    if (n > 1) ICM_CUDA(cudaMemsetAsync(grids[n & 1], 0, grid_bytes, s));
     c->hist_n = n;
     double t = p->SimulationTime;
     for (int k = 1; k <= n; k++) {
         t += p->InitialTimeStep;
         p->indenter_x = p->indenter_x_initial + t * p->IndVelocity;
         icy_SimParams P = kernel_params(c, p);
-        ICM_CUDA(cudaMemsetAsync(c->d_grid, 0, sizeof(double) * c->grid_pitch * ICM_N_GRID_ARRAYS, s));
+        P.grid_array = grids[(n - k) & 1];
+        double *next = k < n && k > 1 ? grids[(n - k + 1) & 1] : nullptr;
+        double *force = c->d_hist + 2 * (size_t)(k - 1);
         const int tp = P.tpb_P2G > 0 ? P.tpb_P2G : 256, tu = P.tpb_Upd > 0 ? P.tpb_Upd : 512;
         const int tg = P.tpb_G2P > 0 ? P.tpb_G2P : 128;
         if (P.nPts > 0) {
-            k_p2g_ref64<<<(P.nPts + tp - 1) / tp, tp, 0, s>>>(P, c->d_err);
-            ICM_LAUNCHED("cuda_p2g");
+            if (k == 1) {
+                k_p2g_ref64<<<(P.nPts + tp - 1) / tp, tp, 0, s>>>(P, c->d_err);
+                ICM_LAUNCHED("cuda_p2g");
+            } else {
+                ICM_CUDA(launch_dependent(s, k_p2g_ref64, (P.nPts + tp - 1) / tp, tp, P, c->d_err));
+            }
         }
-        k_update_ref64<<<(P.GridTotal + tu - 1) / tu, tu, 0, s>>>(P, p->indenter_x, p->indenter_y,
-                                                                  c->d_hist + 2 * (size_t)(k - 1));
-        ICM_LAUNCHED("cuda_update_nodes");
-        if (P.nPts > 0) {
-            k_g2p_ref64<<<(P.nPts + tg - 1) / tg, tg, 0, s>>>(P, (p->SimulationStep + k) % p->UpdateEveryNthStep == 0);
-            ICM_LAUNCHED("cuda_g2p");
-        }
+        ICM_CUDA(launch_dependent(s, k_update_ref64, (P.GridTotal + tu - 1) / tu, tu, P, p->indenter_x, p->indenter_y, force,
+                                  next));
+        if (P.nPts > 0)
+            ICM_CUDA(launch_dependent(s, k_g2p_ref64, (P.nPts + tg - 1) / tg, tg, P,
+                                      (int)((p->SimulationStep + k) % p->UpdateEveryNthStep == 0)));
     }
     p->SimulationStep += n;
     p->SimulationTime = t;
@@ -1048,7 +1079,7 @@ extern "C" int icm_destroy(icm_ctx *c)
     if (c->stream) cudaStreamSynchronize(c->stream);
     free_fused(c);
     free_binning(c);
-    dfree(c->d_pts); dfree(c->d_grid); dfree(c->d_bins); dfree(c->d_err); dfree(c->d_hist); dfree(c->d_redo); dfree(c->d_strays);
+    dfree(c->d_pts); dfree(c->d_grid); dfree(c->d_grid2); dfree(c->d_bins); dfree(c->d_err); dfree(c->d_hist); dfree(c->d_redo); dfree(c->d_strays);
     dfree(c->d_mlp); dfree(c->d_mlp_counts); dfree(c->d_harvest); dfree(c->d_harvest_n);
     if (c->h_ns) cudaFreeHost(c->h_ns);
     if (c->d_tmap) cudaFree(c->d_tmap);
@@ -1124,6 +1155,7 @@ extern "C" int icm_allocate_arrays(icm_ctx *c, icy_SimParams *p, size_t n_grid_n
     ICM_CUDA(cudaStreamSynchronize(c->stream));
     dfree(c->d_pts);
     dfree(c->d_grid);
+    dfree(c->d_grid2);
     dfree(c->d_bins);
     free_fused(c);
     free_binning(c);
@@ -1208,7 +1240,7 @@ extern "C" int icm_update_nodes(icm_ctx *c, double indenter_x, double indenter_y
     if (rc) return rc;
     icy_SimParams P = kernel_params(c, &c->prms);
     int tpb = P.tpb_Upd > 0 ? P.tpb_Upd : 512;
-    k_update_ref64<<<(P.GridTotal + tpb - 1) / tpb, tpb, 0, c->stream>>>(P, indenter_x, indenter_y, nullptr);
+    k_update_ref64<<<(P.GridTotal + tpb - 1) / tpb, tpb, 0, c->stream>>>(P, indenter_x, indenter_y, nullptr, nullptr);
     ICM_LAUNCHED("cuda_update_nodes");
     return ICM_OK;
 }

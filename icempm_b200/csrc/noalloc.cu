@@ -25,9 +25,10 @@
 #include "errors.h"
 
 namespace icm {
-__global__ void k_p2g_ref64(const icy_SimParams P, int *err);
-__global__ void k_update_ref64(const icy_SimParams P, double ind_x, double ind_y, double *force_total);
-__global__ void k_g2p_ref64(const icy_SimParams P, int recordPQ);
+__global__ void k_p2g_ref64(const __grid_constant__ icy_SimParams P, int *err);
+__global__ void k_update_ref64(const __grid_constant__ icy_SimParams P, double ind_x, double ind_y,
+                               double *force_total, double *next);
+__global__ void k_g2p_ref64(const __grid_constant__ icy_SimParams P, int recordPQ);
 }  // namespace icm
 
 namespace {
@@ -111,7 +112,7 @@ extern "C" int icm_run_substeps_noalloc(icy_SimParams *p, double *pts, double *b
         cudaError_t e = cudaMemsetAsync(grid, 0, sizeof(double) * 3 * nodes, s);
         if (e != cudaSuccess) return icm::fail(ICM_ERR_CUDA, std::string("grid clear: ") + cudaGetErrorString(e));
         if (P.nPts > 0) icm::k_p2g_ref64<<<(P.nPts + tp - 1) / tp, tp, 0, s>>>(P, err);
-        icm::k_update_ref64<<<(int)((nodes + tu - 1) / tu), tu, 0, s>>>(P, P.indenter_x, P.indenter_y, nullptr);
+        icm::k_update_ref64<<<(int)((nodes + tu - 1) / tu), tu, 0, s>>>(P, P.indenter_x, P.indenter_y, nullptr, nullptr);
         if (P.nPts > 0)
             icm::k_g2p_ref64<<<(P.nPts + tg - 1) / tg, tg, 0, s>>>(P, (p->SimulationStep + k) % P.UpdateEveryNthStep == 0);
         e = cudaGetLastError();
