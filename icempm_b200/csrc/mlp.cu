@@ -1,17 +1,28 @@
 // mlp.cu -- training and inference of the learned Drucker-Prager projection
 // (mlp.cuh) on the tensor cores.
 //
-// Training: one CTA of 128 threads takes 128 samples (one row per thread,
-// TMEM lane = row) through
+// Training: one CTA takes 128 samples (a row of every tile each, TMEM lane =
+// row) through
 //   forward   Z1 = X W1^T, H1 = gelu(Z1 + b1); Z2 = H1 W2^T, H2 = gelu(..);
 //             Y = H2 W3^T + b3
 //   backward  dZ3 = 2 (Y - T) / (3 B); dH2 = dZ3 W3; dZ2 = dH2 gelu'(..);
 //             dH1 = dZ2 W2; dZ1 = dH1 gelu'(..)
 //   weights   dW3^T = H2^T dZ3, dW2 = dZ2^T H1, dW1 = dZ1^T X
 // with every product a tcgen05 BF16 MMA (M = 128 over samples, M = 64 over
-// hidden units for the weight gradients) accumulating in TMEM; the per-CTA
-// weight gradients go to an FP32 gradient buffer with atomics, and an Adam
-// step (FP32 master weights) follows each batch.
+// hidden units for the weight gradients) accumulating in TMEM; transposed
+// operands are the same tiles read MN-major. The per-CTA gradients go to a
+// slice of an FP32 buffer with plain stores, and an Adam step (FP32 master
+// weights) adds the slices up and writes the next step's BF16 operand tiles.
+// Every sum has a fixed order: training is deterministic.
+//
+// Bound by the latency of the six products and the epilogues between them
+// (TMEM read, bias, GELU, BF16 tiles): 16 warps share the epilogues, a warp
+// taking 16 columns of its quarter of the rows, and keep gelu' in registers
+// for the backward pass. With four warps, transposed copies in 2-byte
+// stores, warp sums of every bias column, atomics and a serial sum over the
+// slices a step of 64 tiles took 78 us (49 this kernel, 9.5 Adam, 5 the
+// operand tiles, a clear and the gaps); now 13.5 + 4.6 us, each launch
+// starting before the one ahead of it ends.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -29,34 +40,37 @@ namespace icm {
 namespace {
 
 // BF16 operand tiles of the tensor-core form, K-major core-matrix layout
-// (tc05.cuh): W1k [64 x 16], W2k [64 x 64], W3k [16 x 64] (rows >= 3 zero),
-// W3Tk [64 x 16] (cols >= 3 zero), W2Tk [64 x 64].
+// (tc05.cuh): W1k [64 x 16], W2k [64 x 64], W3k [16 x 64] (rows >= 3 zero).
 struct MlpTcNet {
-    __nv_bfloat16 W1k[64 * 16], W2k[64 * 64], W3k[16 * 64], W3Tk[64 * 16], W2Tk[64 * 64];
+    __nv_bfloat16 W1k[64 * 16], W2k[64 * 64], W3k[16 * 64];
 };
 
-constexpr int kRows = 128;
+constexpr int kRows = 128, kTileThreads = 4 * kRows;  // rows of a tile; threads (four per row)
+// Floats of a gradient slice: the weights and biases, then the loss, padded
+// so that every slice's rows of W2 start on 16 bytes.
+constexpr int kGradBlocks = kOffXMu / 32 + 1, kSliceFloats = 32 * kGradBlocks;
+static_assert(kOffW2 % 4 == 0);
 // TMEM columns of the accumulators (32-aligned starts). Accumulators share
-// columns where one is dead before the next is written: Z3 is read before
-// dH2 is formed, Z2 (read for gelu' in dH2's epilogue) before dH1, dH2
-// (read in that epilogue) before dW2, dW3^T before dW1; Z1 stays for
-// gelu' of the last step. 256 columns let two CTAs share an SM's 512.
+// columns where one is dead before the next is written: Z1 is read before
+// dH1 is formed, Z3 before dH2, dH2 before dW2, dW3^T before dW1.
 constexpr uint32_t kTmemCols = 256;
-constexpr int cZ1 = 0, cZ2 = 64, cDH1 = 64, cZ3 = 128, cDH2 = 128, cDW2 = 128, cDW3T = 192, cDW1 = 192;
+constexpr int cZ1 = 0, cDH1 = 0, cZ2 = 64, cZ3 = 128, cDH2 = 128, cDW2 = 128, cDW3T = 192, cDW1 = 192;
 constexpr int kWaitPolls = 1 << 24;
 
-// shared-memory layout of k_mlp_tile (bytes). dZ3 takes X's tile (read
-// only by the first product) and dZ2^T takes H2^T's (last read by the
-// product for dW3^T, which completes before dZ2 is formed): 98 KB, two CTAs
-// per SM.
-constexpr int sW1 = 0, sW2 = sW1 + 2048, sW3 = sW2 + 8192, sW3T = sW3 + 2048, sW2T = sW3T + 2048,
-              sX = sW2T + 8192, sXT = sX + 4096, sH1 = sXT + 4096, sH1T = sH1 + 16384, sH2 = sH1T + 16384,
-              sH2T = sH2 + 16384, sDZ3T = sH2T + 16384, kTileSmem = sDZ3T + 4096;
-constexpr int sDZ3 = sX, sDZ2T = sH2T;
+// shared-memory layout of k_mlp_tile (bytes). dZ2 takes H2's tile (last read
+// by the product for dW3^T, which completes before dZ2 is formed) and dZ1
+// H1's.
+constexpr int sW1 = 0, sW2 = sW1 + 2048, sW3 = sW2 + 8192, sX = sW3 + 2048, sH1 = sX + 4096, sH2 = sH1 + 16384,
+              sDZ3 = sH2 + 16384, kTileSmem = sDZ3 + 4096;
 
-__device__ __forceinline__ void put_bf16(unsigned char *base, int row, int k, int K, float v)
+// 16 consecutive columns (c0 a multiple of 16) of a row of a K-major tile
+__device__ __forceinline__ void put_row16(unsigned char *tile, int row, int c0, int cols, const float v[16])
 {
-    *reinterpret_cast<__nv_bfloat16 *>(base + tc05::kmajor_offset(row, k, K)) = __float2bfloat16(v);
+    uint4 a, b;
+    a.x = pack_bf16(v[0], v[1]); a.y = pack_bf16(v[2], v[3]); a.z = pack_bf16(v[4], v[5]); a.w = pack_bf16(v[6], v[7]);
+    b.x = pack_bf16(v[8], v[9]); b.y = pack_bf16(v[10], v[11]); b.z = pack_bf16(v[12], v[13]); b.w = pack_bf16(v[14], v[15]);
+    *reinterpret_cast<uint4 *>(tile + tc05::kmajor_offset(row, c0, cols)) = a;
+    *reinterpret_cast<uint4 *>(tile + tc05::kmajor_offset(row, c0 + 8, cols)) = b;
 }
 
 __device__ __forceinline__ uint32_t sample_index(uint32_t seed, int step, int row, int n)
@@ -68,6 +82,23 @@ __device__ __forceinline__ uint32_t sample_index(uint32_t seed, int step, int ro
     h *= 0x846ca68bu;
     h ^= h >> 16;
     return h % (uint32_t)n;
+}
+
+// The sums over the warp's lanes of 16 values per lane: 16 shuffles, each
+// halving the values a lane still holds. Lane l returns the sum of value
+// (l >> 1) & 15.
+__device__ __forceinline__ float warp_sum16(float v[16], int lane)
+{
+#pragma unroll
+    for (int w = 8; w > 0; w >>= 1) {
+        const bool up = (lane & (2 * w)) != 0;  // this lane keeps the upper half
+#pragma unroll
+        for (int j = 0; j < w; j++) {
+            const float give = up ? v[j] : v[w + j], keep = up ? v[w + j] : v[j];
+            v[j] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * w);
+        }
+    }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
 __device__ __forceinline__ float warp_sum(float v)
@@ -86,58 +117,75 @@ struct TileArgs {
     float inv_count;         // 1 / (3 * samples in the batch)
     const MlpTcNet *tc;      // BF16 operand tiles
     const float *net;        // FP32 parameters (biases, normalisation)
-    float *grad;             // FP32 gradient (same layout as net), accumulated
-    size_t grad_stride;      // CTA b adds into grad + b * grad_stride (0: all into one)
-    float *loss;             // accumulated mean squared error
+    float *grad;             // FP32 gradient slices (net's layout; at kOffXMu the CTA's share of the loss)
+    int first_tile;          // tile of CTA 0 (sequential)
     float *Yout;             // inference: denormalised outputs [n][3]
     int *status;             // set to 1 when a wait gives up
 };
 
+// GELU and its derivative at one point (the tanh form of gelu and gelu_grad)
+__device__ __forceinline__ float gelu_both(float z, float &grad)
+{
+    const float c = 0.7978845608028654f, a = 0.044715f;
+    const float th = tanhf(c * (z + a * z * z * z));
+    grad = 0.5f * (1.0f + th) + 0.5f * z * (1.0f - th * th) * c * (1.0f + 3.0f * a * z * z);
+    return 0.5f * z * (1.0f + th);
+}
+
 template <bool TRAIN>
-__global__ void __launch_bounds__(kRows) k_mlp_tile(const TileArgs a)
+__global__ void __launch_bounds__(kTileThreads, 1) k_mlp_tile(const __grid_constant__ TileArgs a)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t s_tmem;
+    __shared__ float s_bias[2 * kMlpHid + 4];
+    __shared__ float s_db[2][4][kMlpHid], s_db3[4][4];  // bias gradients and loss by quarter of the rows
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // the warp's quarter of the rows (its TMEM lanes) and its 16 columns
+    const int q = warp & 3, c0 = (warp >> 2) * 16, row = q * 32 + lane;
     const float *net = a.net;
-    // this CTA's gradient: its own slice in training, so that the CTAs of a
-    // step do not contend for the same addresses (the Adam step adds the
-    // slices up)
-    float *grad = a.grad + (size_t)blockIdx.x * a.grad_stride;
+    float *grad = a.grad + (size_t)blockIdx.x * kSliceFloats;
 
     // sample of this row
     int idx;
     bool valid;
     if (a.sequential) {
-        idx = blockIdx.x * kRows + tid;
+        idx = (a.first_tile + blockIdx.x) * kRows + row;
         valid = idx < a.n;
     } else {
-        idx = (int)sample_index(a.seed, a.step, blockIdx.x * kRows + tid, a.n);
+        idx = (int)sample_index(a.seed, a.step, blockIdx.x * kRows + row, a.n);
         valid = true;
     }
-    // operand tiles of the weights
+    // normalised inputs and targets: of the network only its normalisation
+    // is read here, which training leaves alone
+    float t[kMlpOut] = {0.f, 0.f, 0.f};
+    if (c0 == 0) {
+        float x[16];
+#pragma unroll
+        for (int k = 0; k < kMlpInPad; k++) {
+            x[k] = 0.f;
+            if (k < kMlpIn && valid) x[k] = (a.X[(size_t)idx * kMlpIn + k] - net[kOffXMu + k]) / net[kOffXSd + k];
+        }
+        put_row16(sm + sX, row, 0, 16, x);
+        if (TRAIN && valid)
+#pragma unroll
+            for (int o = 0; o < kMlpOut; o++) t[o] = (a.Y[(size_t)idx * kMlpOut + o] - net[kOffYMu + o]) / net[kOffYSd + o];
+    }
+    if (tid == 0) tc05::mbar_init(&mbar, 1);
+    if (warp == 0) tc05::alloc(&s_tmem, kTmemCols);
+    // in training a programmatic dependent of the Adam step before
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // operand tiles of the weights, biases
     {
         const uint4 *src = reinterpret_cast<const uint4 *>(a.tc);
         uint4 *dst = reinterpret_cast<uint4 *>(sm + sW1);
         const int nvec = (int)(sizeof(MlpTcNet) / 16);
-        for (int i = tid; i < nvec; i += kRows) dst[i] = src[i];
+        for (int i = tid; i < nvec; i += kTileThreads) dst[i] = src[i];
+        if (tid < kMlpHid) s_bias[tid] = net[kOffB1 + tid];
+        else if (tid < 2 * kMlpHid) s_bias[tid] = net[kOffB2 + tid - kMlpHid];
+        else if (tid < 2 * kMlpHid + kMlpOut) s_bias[tid] = net[kOffB3 + tid - 2 * kMlpHid];
     }
-    // normalised inputs: row tid of X, column tid of X^T
-#pragma unroll
-    for (int k = 0; k < kMlpInPad; k++) {
-        float v = 0.f;
-        if (k < kMlpIn && valid) v = (a.X[(size_t)idx * kMlpIn + k] - net[kOffXMu + k]) / net[kOffXSd + k];
-        put_bf16(sm + sX, tid, k, 16, v);
-        if (TRAIN) put_bf16(sm + sXT, k, tid, kRows, v);
-    }
-    if (tid == 0) tc05::mbar_init(&mbar, 1);
-    if (warp == 0) tc05::alloc(&s_tmem, kTmemCols);
-    tc05::fence_smem_for_mma();
-    tc05::fence_before_sync();
-    __syncthreads();
-    tc05::fence_after_sync();
-    const uint32_t tmem = s_tmem;
     uint32_t phase = 0;
     bool ok = true;
     auto wait_mma = [&]() {
@@ -151,8 +199,14 @@ __global__ void __launch_bounds__(kRows) k_mlp_tile(const TileArgs a)
         __syncthreads();
         tc05::fence_after_sync();
     };
-    const uint32_t id128x64 = tc05::idesc_bf16(128, 64), id128x16 = tc05::idesc_bf16(128, 16);
-    const uint32_t id64x16 = tc05::idesc_bf16(64, 16), id64x64 = tc05::idesc_bf16(64, 64);
+    publish();
+    const uint32_t tmem = s_tmem;
+    constexpr uint32_t id128x64 = tc05::idesc_bf16(128, 64), id128x16 = tc05::idesc_bf16(128, 16);
+    constexpr uint32_t id128x64t = tc05::idesc_bf16(128, 64, false, true);  // B read transposed
+    constexpr uint32_t id64x16tt = tc05::idesc_bf16(64, 16, true, true), id64x64tt = tc05::idesc_bf16(64, 64, true, true);
+    // bytes to the next K = 16 of a tile of 64 / 16 columns: along a row, down the rows
+    constexpr int kAlong = 256, kDown64 = 2048, kDown16 = 512;
+    float z[16], d1[16], d2[16];
 
     // ---- Z1 = X W1^T
     if (tid == 0) {
@@ -160,147 +214,139 @@ __global__ void __launch_bounds__(kRows) k_mlp_tile(const TileArgs a)
         tc05::commit(&mbar);
     }
     wait_mma();
-    float z[16];
-#pragma unroll 1
-    for (int c0 = 0; c0 < 64; c0 += 16) {
-        tc05::ld16(tc05::taddr(tmem, warp, cZ1 + c0), z);
+    tc05::ld16(tc05::taddr(tmem, q, cZ1 + c0), z);
 #pragma unroll
-        for (int j = 0; j < 16; j++) {
-            const float h = gelu(z[j] + net[kOffB1 + c0 + j]);
-            put_bf16(sm + sH1, tid, c0 + j, 64, h);
-            if (TRAIN) put_bf16(sm + sH1T, c0 + j, tid, kRows, h);
-        }
-    }
+    for (int j = 0; j < 16; j++) z[j] = TRAIN ? gelu_both(z[j] + s_bias[c0 + j], d1[j]) : gelu(z[j] + s_bias[c0 + j]);
+    put_row16(sm + sH1, row, c0, 64, z);
     publish();
     // ---- Z2 = H1 W2^T
     if (tid == 0) {
         for (int kk = 0; kk < 4; kk++)
-            tc05::mma(tmem + cZ2, tc05::desc_kmajor(sm + sH1 + 256 * kk, 64), tc05::desc_kmajor(sm + sW2 + 256 * kk, 64),
-                      id128x64, kk > 0);
+            tc05::mma(tmem + cZ2, tc05::desc_kmajor(sm + sH1 + kAlong * kk, 64),
+                      tc05::desc_kmajor(sm + sW2 + kAlong * kk, 64), id128x64, kk > 0);
         tc05::commit(&mbar);
     }
     wait_mma();
-#pragma unroll 1
-    for (int c0 = 0; c0 < 64; c0 += 16) {
-        tc05::ld16(tc05::taddr(tmem, warp, cZ2 + c0), z);
+    tc05::ld16(tc05::taddr(tmem, q, cZ2 + c0), z);
 #pragma unroll
-        for (int j = 0; j < 16; j++) {
-            const float h = gelu(z[j] + net[kOffB2 + c0 + j]);
-            put_bf16(sm + sH2, tid, c0 + j, 64, h);
-            if (TRAIN) put_bf16(sm + sH2T, c0 + j, tid, kRows, h);
-        }
-    }
+    for (int j = 0; j < 16; j++)
+        z[j] = TRAIN ? gelu_both(z[j] + s_bias[kMlpHid + c0 + j], d2[j]) : gelu(z[j] + s_bias[kMlpHid + c0 + j]);
+    put_row16(sm + sH2, row, c0, 64, z);
     publish();
     // ---- Y = H2 W3^T + b3
     if (tid == 0) {
         for (int kk = 0; kk < 4; kk++)
-            tc05::mma(tmem + cZ3, tc05::desc_kmajor(sm + sH2 + 256 * kk, 64), tc05::desc_kmajor(sm + sW3 + 256 * kk, 64),
-                      id128x16, kk > 0);
+            tc05::mma(tmem + cZ3, tc05::desc_kmajor(sm + sH2 + kAlong * kk, 64),
+                      tc05::desc_kmajor(sm + sW3 + kAlong * kk, 64), id128x16, kk > 0);
         tc05::commit(&mbar);
     }
     wait_mma();
-    tc05::ld16(tc05::taddr(tmem, warp, cZ3), z);
-    float y[kMlpOut];
+    if (c0 == 0) {
+        tc05::ld16(tc05::taddr(tmem, q, cZ3), z);
+        float y[kMlpOut];
 #pragma unroll
-    for (int o = 0; o < kMlpOut; o++) y[o] = z[o] + net[kOffB3 + o];
-
-    if (!TRAIN) {
-        if (valid)
-            for (int o = 0; o < kMlpOut; o++)
-                a.Yout[(size_t)idx * kMlpOut + o] = y[o] * net[kOffYSd + o] + net[kOffYMu + o];
-    } else {
-        // ---- loss and dZ3
-        float dy[kMlpOut], se = 0.f;
+        for (int o = 0; o < kMlpOut; o++) y[o] = z[o] + s_bias[2 * kMlpHid + o];
+        if (!TRAIN) {
+            if (valid)
+                for (int o = 0; o < kMlpOut; o++)
+                    a.Yout[(size_t)idx * kMlpOut + o] = y[o] * net[kOffYSd + o] + net[kOffYMu + o];
+        } else {
+            // ---- loss and dZ3
+            float dy[16], se = 0.f;
 #pragma unroll
-        for (int o = 0; o < kMlpOut; o++) {
-            const float t = valid ? (a.Y[(size_t)idx * kMlpOut + o] - net[kOffYMu + o]) / net[kOffYSd + o] : y[o];
-            const float d = y[o] - t;
-            se += d * d;
-            dy[o] = valid ? 2.f * d * a.inv_count : 0.f;
+            for (int o = 0; o < 16; o++) {
+                dy[o] = 0.f;
+                if (o < kMlpOut && valid) {
+                    const float d = y[o] - t[o];
+                    se += d * d;
+                    dy[o] = 2.f * d * a.inv_count;
+                }
+            }
+            put_row16(sm + sDZ3, row, 0, 16, dy);
+            se = warp_sum(se);
+#pragma unroll
+            for (int o = 0; o < kMlpOut; o++) dy[o] = warp_sum(dy[o]);
+            if (lane == 0) {
+#pragma unroll
+                for (int o = 0; o < kMlpOut; o++) s_db3[q][o] = dy[o];
+                s_db3[q][3] = se * a.inv_count;
+            }
         }
-#pragma unroll
-        for (int o = 0; o < 16; o++) {
-            const float v = o < kMlpOut ? dy[o] : 0.f;
-            put_bf16(sm + sDZ3, tid, o, 16, v);
-            put_bf16(sm + sDZ3T, o, tid, kRows, v);
-        }
-        se = warp_sum(se);
-        if (lane == 0) atomicAdd(a.loss, se * a.inv_count);
-#pragma unroll
-        for (int o = 0; o < kMlpOut; o++) {
-            const float s = warp_sum(dy[o]);
-            if (lane == 0) atomicAdd(&grad[kOffB3 + o], s);
-        }
+    }
+    if (TRAIN) {
         publish();
         // ---- dH2 = dZ3 W3 ; dW3^T = H2^T dZ3
         if (tid == 0) {
-            tc05::mma(tmem + cDH2, tc05::desc_kmajor(sm + sDZ3, 16), tc05::desc_kmajor(sm + sW3T, 16), id128x64, false);
+            tc05::mma(tmem + cDH2, tc05::desc_kmajor(sm + sDZ3, 16), tc05::desc_mnmajor(sm + sW3, 64), id128x64t, false);
             for (int kk = 0; kk < 8; kk++)
-                tc05::mma(tmem + cDW3T, tc05::desc_kmajor(sm + sH2T + 256 * kk, kRows),
-                          tc05::desc_kmajor(sm + sDZ3T + 256 * kk, kRows), id64x16, kk > 0);
+                tc05::mma(tmem + cDW3T, tc05::desc_mnmajor(sm + sH2 + kDown64 * kk, 64),
+                          tc05::desc_mnmajor(sm + sDZ3 + kDown16 * kk, 16), id64x16tt, kk > 0);
             tc05::commit(&mbar);
         }
-        wait_mma();
-        float dh[16];
-#pragma unroll 1
-        for (int c0 = 0; c0 < 64; c0 += 16) {
-            tc05::ld16(tc05::taddr(tmem, warp, cDH2 + c0), dh);
-            tc05::ld16(tc05::taddr(tmem, warp, cZ2 + c0), z);
-#pragma unroll
-            for (int j = 0; j < 16; j++) {
-                const float d = dh[j] * gelu_grad(z[j] + net[kOffB2 + c0 + j]);
-                put_bf16(sm + sH2, tid, c0 + j, 64, d);  // dZ2 over H2 (no longer read)
-                put_bf16(sm + sDZ2T, c0 + j, tid, kRows, d);
-                const float s = warp_sum(d);
-                if (lane == 0) atomicAdd(&grad[kOffB2 + c0 + j], s);
-            }
+        if (tid < kMlpOut + 1) {
+            const float s = s_db3[0][tid] + s_db3[1][tid] + s_db3[2][tid] + s_db3[3][tid];
+            grad[tid < kMlpOut ? kOffB3 + tid : kOffXMu] = s;
         }
-        // dW3^T rows (hidden unit 16 warp + lane for lanes < 16)
-        tc05::ld16(tc05::taddr(tmem, warp, cDW3T), dh);
-        if (lane < 16)
-            for (int o = 0; o < kMlpOut; o++) atomicAdd(&grad[kOffW3 + o * kMlpHid + warp * 16 + lane], dh[o]);
+        wait_mma();
+        tc05::ld16(tc05::taddr(tmem, q, cDH2 + c0), z);
+#pragma unroll
+        for (int j = 0; j < 16; j++) z[j] *= d2[j];
+        put_row16(sm + sH2, row, c0, 64, z);  // dZ2 over H2 (no longer read)
+        {
+            const float s = warp_sum16(z, lane);
+            if ((lane & 1) == 0) s_db[1][q][c0 + (lane >> 1)] = s;
+        }
+        // dW3^T rows (hidden unit 16 q + lane for lanes < 16)
+        if (c0 == 0) {
+            tc05::ld16(tc05::taddr(tmem, q, cDW3T), z);
+            if (lane < 16)
+                for (int o = 0; o < kMlpOut; o++) grad[kOffW3 + o * kMlpHid + q * 16 + lane] = z[o];
+        }
         publish();
         // ---- dH1 = dZ2 W2 ; dW2 = dZ2^T H1
         if (tid == 0) {
             for (int kk = 0; kk < 4; kk++)
-                tc05::mma(tmem + cDH1, tc05::desc_kmajor(sm + sH2 + 256 * kk, 64),
-                          tc05::desc_kmajor(sm + sW2T + 256 * kk, 64), id128x64, kk > 0);
+                tc05::mma(tmem + cDH1, tc05::desc_kmajor(sm + sH2 + kAlong * kk, 64),
+                          tc05::desc_mnmajor(sm + sW2 + kDown64 * kk, 64), id128x64t, kk > 0);
             for (int kk = 0; kk < 8; kk++)
-                tc05::mma(tmem + cDW2, tc05::desc_kmajor(sm + sDZ2T + 256 * kk, kRows),
-                          tc05::desc_kmajor(sm + sH1T + 256 * kk, kRows), id64x64, kk > 0);
+                tc05::mma(tmem + cDW2, tc05::desc_mnmajor(sm + sH2 + kDown64 * kk, 64),
+                          tc05::desc_mnmajor(sm + sH1 + kDown64 * kk, 64), id64x64tt, kk > 0);
             tc05::commit(&mbar);
         }
         wait_mma();
-#pragma unroll 1
-        for (int c0 = 0; c0 < 64; c0 += 16) {
-            tc05::ld16(tc05::taddr(tmem, warp, cDH1 + c0), dh);
-            tc05::ld16(tc05::taddr(tmem, warp, cZ1 + c0), z);
+        tc05::ld16(tc05::taddr(tmem, q, cDH1 + c0), z);
 #pragma unroll
-            for (int j = 0; j < 16; j++) {
-                const float d = dh[j] * gelu_grad(z[j] + net[kOffB1 + c0 + j]);
-                put_bf16(sm + sH1, c0 + j, tid, kRows, d);  // dZ1^T over H1 (no longer read)
-                const float s = warp_sum(d);
-                if (lane == 0) atomicAdd(&grad[kOffB1 + c0 + j], s);
-            }
-        }
-#pragma unroll 1
-        for (int c0 = 0; c0 < 64; c0 += 16) {
-            tc05::ld16(tc05::taddr(tmem, warp, cDW2 + c0), dh);
-            if (lane < 16)
-                for (int j = 0; j < 16; j++) atomicAdd(&grad[kOffW2 + (warp * 16 + lane) * kMlpHid + c0 + j], dh[j]);
+        for (int j = 0; j < 16; j++) z[j] *= d1[j];
+        put_row16(sm + sH1, row, c0, 64, z);  // dZ1 over H1 (no longer read)
+        {
+            const float s = warp_sum16(z, lane);
+            if ((lane & 1) == 0) s_db[0][q][c0 + (lane >> 1)] = s;
         }
         publish();
         // ---- dW1 = dZ1^T X
         if (tid == 0) {
             for (int kk = 0; kk < 8; kk++)
-                tc05::mma(tmem + cDW1, tc05::desc_kmajor(sm + sH1 + 256 * kk, kRows),
-                          tc05::desc_kmajor(sm + sXT + 256 * kk, kRows), id64x16, kk > 0);
+                tc05::mma(tmem + cDW1, tc05::desc_mnmajor(sm + sH1 + kDown64 * kk, 64),
+                          tc05::desc_mnmajor(sm + sX + kDown16 * kk, 16), id64x16tt, kk > 0);
             tc05::commit(&mbar);
         }
+        // meanwhile dW2 (columns 128-191) and the bias gradients
+        tc05::ld16(tc05::taddr(tmem, q, cDW2 + c0), z);
+        if (lane < 16) {
+            float4 *w = reinterpret_cast<float4 *>(grad + kOffW2 + (q * 16 + lane) * kMlpHid + c0);
+#pragma unroll
+            for (int j = 0; j < 4; j++) w[j] = make_float4(z[4 * j], z[4 * j + 1], z[4 * j + 2], z[4 * j + 3]);
+        }
+        if (tid < 2 * kMlpHid) {
+            const int l = tid >> 6, u = tid & 63;
+            grad[(l ? kOffB2 : kOffB1) + u] = s_db[l][0][u] + s_db[l][1][u] + s_db[l][2][u] + s_db[l][3][u];
+        }
         wait_mma();
-        tc05::ld16(tc05::taddr(tmem, warp, cDW1), dh);
-        if (lane < 16)
-            for (int i = 0; i < kMlpIn; i++) atomicAdd(&grad[kOffW1 + (warp * 16 + lane) * kMlpIn + i], dh[i]);
+        if (c0 == 0) {
+            tc05::ld16(tc05::taddr(tmem, q, cDW1), z);
+            if (lane < 16)
+                for (int i = 0; i < kMlpIn; i++) grad[kOffW1 + (q * 16 + lane) * kMlpIn + i] = z[i];
+        }
     }
     if (!ok && a.status) atomicExch(a.status, 1);
     tc05::fence_before_sync();
@@ -323,18 +369,16 @@ __global__ void k_mlp_prep(const float *net, MlpTcNet *tc, MlpWarpNet *wn)
         put(tc->W1k, o, k, 16, w);
         if (wn) wn->W1[o * 16 + k] = __float2bfloat16(w);
     }
-    if (i < 64 * 64) {  // W2 [64][64] and its transpose
+    if (i < 64 * 64) {  // W2 [64][64]
         const int o = i / 64, k = i % 64;
         const float w = net[kOffW2 + o * 64 + k];
         put(tc->W2k, o, k, 64, w);
-        put(tc->W2Tk, k, o, 64, w);
         if (wn) wn->W2[o * 64 + k] = __float2bfloat16(w);
     }
-    if (i < 16 * 64) {  // W3 [16][64] (3 real rows) and its transpose [64][16]
+    if (i < 16 * 64) {  // W3 [16][64] (3 real rows)
         const int o = i / 64, k = i % 64;
         const float w = o < kMlpOut ? net[kOffW3 + o * 64 + k] : 0.f;
         put(tc->W3k, o, k, 64, w);
-        put(tc->W3Tk, k, o, 16, w);
         if (wn && o < 8) wn->W3[o * 64 + k] = __float2bfloat16(w);
     }
     if (wn && i < 64) {
@@ -352,19 +396,66 @@ __global__ void k_mlp_prep(const float *net, MlpTcNet *tc, MlpWarpNet *wn)
     }
 }
 
-// Adam on the weights and biases (not the normalisation)
-// Adam step on the sum of nslices gradient slices (stride floats apart)
-__global__ void k_mlp_adam(float *net, float *m, float *v, const float *grad, int nslices, size_t stride, int count,
-                           float lr, float b1, float b2, float eps, float c1, float c2)
+// The sum of nslices gradient slices for the 32 parameters of a block: eight
+// warps share the slices (coalesced rows of 32), their sums are added in a
+// fixed order and returned in warp 0. (One thread per parameter over all 64
+// slices took 9.5 us, waiting for one load after another.)
+constexpr int kSumWarps = 8;
+__device__ __forceinline__ float slice_sum(const float *grad, int nslices, int i, bool on)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
+    __shared__ float s_part[kSumWarps][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     float g = 0.f;
-    for (int b = 0; b < nslices; b++) g += grad[(size_t)b * stride + i];
+    if (on) {
+#pragma unroll 8
+        for (int b = w; b < nslices; b += kSumWarps) g += grad[(size_t)b * kSliceFloats + i];
+    }
+    s_part[w][lane] = g;
+    __syncthreads();
+    g = 0.f;
+    if (w == 0) {
+#pragma unroll
+        for (int k = 0; k < kSumWarps; k++) g += s_part[k][lane];
+    }
+    return g;
+}
+
+// Adam step on the weights and biases (not the normalisation) with the sum
+// of the gradient slices; writes the BF16 operand tiles of the next step
+// (their padding stays as k_mlp_prep left it) and the step's loss.
+__global__ void __launch_bounds__(32 * kSumWarps) k_mlp_adam(float *net, float *m, float *v, const float *grad, int nslices,
+                                                            MlpTcNet *tc, float *loss, float lr, float b1, float b2,
+                                                            float eps, float c1, float c2)
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31);
+    const float g = slice_sum(grad, nslices, i, i <= kOffXMu);
+    if (threadIdx.x >= 32 || i > kOffXMu) return;
+    if (i == kOffXMu) {
+        *loss = g;
+        return;
+    }
     const float mi = b1 * m[i] + (1.f - b1) * g, vi = b2 * v[i] + (1.f - b2) * g * g;
     m[i] = mi;
     v[i] = vi;
-    net[i] -= lr * (mi * c1) / (sqrtf(vi * c2) + eps);
+    const float w = net[i] - lr * (mi * c1) / (sqrtf(vi * c2) + eps);
+    net[i] = w;
+    auto put = [&](__nv_bfloat16 *tile, int row, int k, int K) {
+        *reinterpret_cast<__nv_bfloat16 *>(reinterpret_cast<unsigned char *>(tile) + tc05::kmajor_offset(row, k, K)) =
+            __float2bfloat16(w);
+    };
+    if (i < kOffB1) put(tc->W1k, (i - kOffW1) / kMlpIn, (i - kOffW1) % kMlpIn, 16);
+    else if (i >= kOffW2 && i < kOffB2) put(tc->W2k, (i - kOffW2) / 64, (i - kOffW2) % 64, 64);
+    else if (i >= kOffW3 && i < kOffB3) put(tc->W3k, (i - kOffW3) / 64, (i - kOffW3) % 64, 64);
+}
+
+// Adds the sum of the gradient slices to sum (kOffXMu: the loss).
+__global__ void __launch_bounds__(32 * kSumWarps) k_mlp_sum(float *sum, const float *grad, int nslices)
+{
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31);
+    const float g = slice_sum(grad, nslices, i, i <= kOffXMu);
+    if (threadIdx.x < 32 && i <= kOffXMu) sum[i] += g;
 }
 
 // the warp form over a batch (tests and measurements of the in-kernel form)
@@ -419,6 +510,39 @@ template <class T> struct DevBuf {
                    : icm::fail(ICM_ERR_NOMEM, "mlp: device allocation failed");
     }
 };
+
+struct Stream {
+    cudaStream_t s = nullptr;
+    ~Stream()
+    {
+        if (s) cudaStreamDestroy(s);
+    }
+    int create()
+    {
+        return cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess
+                   ? ICM_OK
+                   : icm::fail(ICM_ERR_CUDA, "mlp: stream");
+    }
+};
+
+// a launch that may start before the kernel ahead of it on the stream ends
+// (dependent; the kernels wait for it themselves)
+template <class... KArgs, class... Args>
+cudaError_t launch_next(cudaStream_t s, bool dependent, void (*kernel)(KArgs...), int blocks, int threads, size_t smem,
+                        Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = dependent ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
 
 // the opt-in is per device (cudaFuncSetAttribute acts on the current one)
 int set_tile_smem()
@@ -527,11 +651,12 @@ extern "C" int icm_mlp_train(int device, const float *x, const float *y, int n, 
     DevBuf<float> X, Y, net, m, v, grad, loss;
     DevBuf<MlpTcNet> tc;
     DevBuf<int> status;
+    Stream stream;
     const int steps = cfg->steps;
     if ((rc = X.alloc((size_t)n * kMlpIn)) || (rc = Y.alloc((size_t)n * kMlpOut)) || (rc = net.alloc(kMlpFloats)) ||
         (rc = m.alloc(kMlpFloats)) || (rc = v.alloc(kMlpFloats)) ||
-        (rc = grad.alloc((size_t)std::max(cfg->batch_tiles, 1) * kMlpFloats)) ||
-        (rc = loss.alloc(std::max(steps, 1))) || (rc = tc.alloc(1)) || (rc = status.alloc(1)))
+        (rc = grad.alloc((size_t)std::max(cfg->batch_tiles, 1) * kSliceFloats)) ||
+        (rc = loss.alloc(std::max(steps, 1))) || (rc = tc.alloc(1)) || (rc = status.alloc(1)) || (rc = stream.create()))
         return rc;
     cudaMemcpy(X.p, x, sizeof(float) * n * kMlpIn, cudaMemcpyHostToDevice);
     cudaMemcpy(Y.p, y, sizeof(float) * n * kMlpOut, cudaMemcpyHostToDevice);
@@ -551,21 +676,22 @@ extern "C" int icm_mlp_train(int device, const float *x, const float *y, int n, 
     a.tc = tc.p;
     a.net = net.p;
     a.grad = grad.p;
-    a.grad_stride = kMlpFloats;
     a.status = status.p;
-    const int nw = kOffXMu;  // weights and biases
+    // the default stream's copies and clears first: the steps run on a stream
+    // of their own, each launch a programmatic dependent of the one before
+    if (cudaStreamSynchronize(0) != cudaSuccess) return icm::fail(ICM_ERR_CUDA, "icm_mlp_train: set-up");
+    launch_prep(net.p, tc.p, nullptr, stream.s);
     for (int s = 0; s < steps; s++) {
-        launch_prep(net.p, tc.p, nullptr);
-        cudaMemsetAsync(grad.p, 0, sizeof(float) * kMlpFloats * (size_t)cfg->batch_tiles);
         a.step = s;
-        a.loss = loss.p + s;
-        k_mlp_tile<true><<<cfg->batch_tiles, kRows, kTileSmem>>>(a);
+        const cudaError_t e1 = launch_next(stream.s, s > 0, k_mlp_tile<true>, cfg->batch_tiles, kTileThreads, kTileSmem, a);
+        if (e1 != cudaSuccess) return icm::fail(ICM_ERR_CUDA, std::string("icm_mlp_train: ") + cudaGetErrorString(e1));
         // cosine decay from lr to lr/20
         const float frac = steps > 1 ? (float)s / (float)(steps - 1) : 0.f;
         const float lr = cfg->lr * (0.05f + 0.95f * 0.5f * (1.0f + std::cos(3.14159265f * frac)));
         const float c1 = 1.0f / (1.0f - std::pow(b1, (float)(s + 1))), c2 = 1.0f / (1.0f - std::pow(b2, (float)(s + 1)));
-        k_mlp_adam<<<(nw + 255) / 256, 256>>>(net.p, m.p, v.p, grad.p, cfg->batch_tiles, kMlpFloats, nw, lr, b1, b2,
-                                              eps, c1, c2);
+        const cudaError_t e2 = launch_next(stream.s, true, k_mlp_adam, kGradBlocks, 32 * kSumWarps, 0, net.p, m.p, v.p,
+                                           (const float *)grad.p, cfg->batch_tiles, tc.p, loss.p + s, lr, b1, b2, eps, c1, c2);
+        if (e2 != cudaSuccess) return icm::fail(ICM_ERR_CUDA, std::string("icm_mlp_train: ") + cudaGetErrorString(e2));
     }
     if ((rc = finish_device("icm_mlp_train", status.p))) return rc;
     cudaMemcpy(net_io, net.p, sizeof(float) * kMlpFloats, cudaMemcpyDeviceToHost);
@@ -579,17 +705,18 @@ extern "C" int icm_mlp_gradient(int device, const float *net_in, const float *x,
     if (!net_in || !x || !y || !grad_out || n < 1) return icm::fail(ICM_ERR_ARG, "icm_mlp_gradient: bad arguments");
     int rc = select_device(device);
     if (rc || (rc = set_tile_smem())) return rc;
-    DevBuf<float> X, Y, net, grad, loss;
+    DevBuf<float> X, Y, net, grad, sum;
     DevBuf<MlpTcNet> tc;
     DevBuf<int> status;
+    const int tiles = (n + kRows - 1) / kRows, kSlices = 1024;  // tiles per launch
     if ((rc = X.alloc((size_t)n * kMlpIn)) || (rc = Y.alloc((size_t)n * kMlpOut)) || (rc = net.alloc(kMlpFloats)) ||
-        (rc = grad.alloc(kMlpFloats)) || (rc = loss.alloc(1)) || (rc = tc.alloc(1)) || (rc = status.alloc(1)))
+        (rc = grad.alloc((size_t)std::min(tiles, kSlices) * kSliceFloats)) || (rc = sum.alloc(kMlpFloats)) || (rc = tc.alloc(1)) ||
+        (rc = status.alloc(1)))
         return rc;
     cudaMemcpy(X.p, x, sizeof(float) * n * kMlpIn, cudaMemcpyHostToDevice);
     cudaMemcpy(Y.p, y, sizeof(float) * n * kMlpOut, cudaMemcpyHostToDevice);
     cudaMemcpy(net.p, net_in, sizeof(float) * kMlpFloats, cudaMemcpyHostToDevice);
-    cudaMemset(grad.p, 0, sizeof(float) * kMlpFloats);
-    cudaMemset(loss.p, 0, sizeof(float));
+    cudaMemset(sum.p, 0, sizeof(float) * kMlpFloats);
     cudaMemset(status.p, 0, sizeof(int));
     launch_prep(net.p, tc.p, nullptr);
     TileArgs a{};
@@ -601,12 +728,17 @@ extern "C" int icm_mlp_gradient(int device, const float *net_in, const float *x,
     a.tc = tc.p;
     a.net = net.p;
     a.grad = grad.p;
-    a.loss = loss.p;
     a.status = status.p;
-    k_mlp_tile<true><<<(n + kRows - 1) / kRows, kRows, kTileSmem>>>(a);
+    for (a.first_tile = 0; a.first_tile < tiles; a.first_tile += kSlices) {
+        const int k = std::min(tiles - a.first_tile, kSlices);
+        k_mlp_tile<true><<<k, kTileThreads, kTileSmem>>>(a);
+        k_mlp_sum<<<kGradBlocks, 32 * kSumWarps>>>(sum.p, grad.p, k);
+    }
     if ((rc = finish_device("icm_mlp_gradient", status.p))) return rc;
-    cudaMemcpy(grad_out, grad.p, sizeof(float) * kMlpFloats, cudaMemcpyDeviceToHost);
-    if (loss_out) cudaMemcpy(loss_out, loss.p, sizeof(float), cudaMemcpyDeviceToHost);
+    float loss = 0.f;
+    cudaMemcpy(grad_out, sum.p, sizeof(float) * kMlpFloats, cudaMemcpyDeviceToHost);
+    std::swap(loss, grad_out[kOffXMu]);  // the normalisation has no gradient
+    if (loss_out) *loss_out = loss;
     return ICM_OK;
 }
 
@@ -637,7 +769,7 @@ extern "C" int icm_mlp_infer(int device, const float *net_in, const float *x, in
         a.net = net.p;
         a.Yout = Yo.p;
         a.status = status.p;
-        k_mlp_tile<false><<<(n + kRows - 1) / kRows, kRows, kTileSmem>>>(a);
+        k_mlp_tile<false><<<(n + kRows - 1) / kRows, kTileThreads, kTileSmem>>>(a);
     }
     if ((rc = finish_device("icm_mlp_infer", status.p))) return rc;
     cudaMemcpy(y_out, Yo.p, sizeof(float) * n * kMlpOut, cudaMemcpyDeviceToHost);

@@ -10,6 +10,13 @@
 // stride-byte offset (next 8 rows) is (K/8) * 128. One MMA consumes K = 16;
 // the next 16 columns start 256 bytes further on.
 //
+// The same tile is also read with its columns as the M or N dimension and its
+// rows as K (MN-major), so that a product with a transpose needs no
+// transposed copy: a core matrix then is 8 K-rows of 8 contiguous M/N
+// elements, the stride-byte offset (next 8 of M/N) is 128 and the
+// leading-byte offset (next 8 of K) is (columns/8) * 128. The next K = 16
+// rows start twice that further on.
+//
 // Accumulators live in tensor memory: for M = 128, row m is lane m; for
 // M = 64, row m is lane (m % 16) + 32 * (m / 16), i.e. the first 16 lanes of
 // each warp's quarter. tcgen05.ld.32x32b gives thread t of warp w lane
@@ -39,10 +46,25 @@ __device__ __forceinline__ uint64_t desc_kmajor(const void *tile, int K)
     return d;
 }
 
-// instruction descriptor: BF16 A and B, FP32 accumulator, both K-major
-__host__ __device__ constexpr uint32_t idesc_bf16(int M, int N)
+// shared-memory matrix descriptor: MN-major, no swizzle, of a tile of `cols`
+// columns (the M or N dimension)
+__device__ __forceinline__ uint64_t desc_mnmajor(const void *tile, int cols)
 {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+    const uint32_t addr = smem_u32(tile);
+    const uint32_t lbo = (uint32_t)(cols >> 3) * 128, sbo = 128;
+    uint64_t d = (uint64_t)((addr >> 4) & 0x3fff);
+    d |= (uint64_t)((lbo >> 4) & 0x3fff) << 16;
+    d |= (uint64_t)((sbo >> 4) & 0x3fff) << 32;
+    d |= (uint64_t)1 << 46;  // descriptor version of sm_100
+    return d;
+}
+
+// instruction descriptor: BF16 A and B, FP32 accumulator; ta, tb: A, B are
+// MN-major
+__host__ __device__ constexpr uint32_t idesc_bf16(int M, int N, bool ta = false, bool tb = false)
+{
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)ta << 15) | ((uint32_t)tb << 16) |
+           ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
 // D[tmem] (+)= A * B^T for one K = 16 slice; issued by one thread
