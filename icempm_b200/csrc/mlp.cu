@@ -22,7 +22,8 @@
 // stores, warp sums of every bias column, atomics and a serial sum over the
 // slices a step of 64 tiles took 78 us (49 this kernel, 9.5 Adam, 5 the
 // operand tiles, a clear and the gaps); now 13.5 + 4.6 us, each launch
-// starting before the one ahead of it ends.
+// starting before the one ahead of it ends. Two CTAs fit an SM: 296 tiles a
+// step 18.7 us (one CTA 21.8, before 74).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -133,7 +134,7 @@ __device__ __forceinline__ float gelu_both(float z, float &grad)
 }
 
 template <bool TRAIN>
-__global__ void __launch_bounds__(kTileThreads, 1) k_mlp_tile(const __grid_constant__ TileArgs a)
+__global__ void __launch_bounds__(kTileThreads, 2) k_mlp_tile(const __grid_constant__ TileArgs a)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ __align__(8) uint64_t mbar;
