@@ -97,9 +97,10 @@ struct Fused {
 
 }  // namespace
 
-// the last answer of pair_threads and what it was for
-struct PairThreads {
+// the last answer of widened_threads and what it was for
+struct WideThreads {
     int threads = 0, nbusy = -1, cells = 0, answer = 0;
+    const void *kernel = nullptr;
 };
 
 struct icm_ctx {
@@ -151,7 +152,7 @@ struct icm_ctx {
     int nslots = 0;
     int *h_ns = nullptr;  // pinned: the slot count and busy tiles a re-binning reads back
     int nbusy = 0;        // tiles holding particles in the current binning
-    PairThreads wide;     // threads of the fused launches (pair_threads)
+    WideThreads wide;     // threads of the fused launches (widened_threads)
     // TMA descriptors of the three grid buffers (device copy) and what they
     // were encoded for
     CUtensorMap *d_tmap = nullptr;
@@ -520,19 +521,29 @@ static void opted_in(size_t *opted, int device, size_t dyn)
 // more warps than a tile has groups of 32 cells, and as many for each
 static bool pair_wide(int cells, int threads) { return threads > cells && threads % cells == 0; }
 
-// the pair loop's static shared memory (the lists of at most 16 groups), and room for the rest
-constexpr size_t kPairStaticBytes = 16 * (384 + 8) + 1024;
+// Forms whose full substep runs with more threads than asked for when the
+// tiles are few: the pair loop up to 16 warps a tile, two per group of cells;
+// the FP64 loop up to a warp per group (its 168 registers fill an SM at 384
+// threads). The surrogate form has staging for four warps.
+template <class Pol, int MODE>
+constexpr bool kWidens = kPairLaunch<Pol, MODE> || (std::is_same<Pol, Pol64>::value && MODE == kModeFull);
+template <class Pol> constexpr int kWidestThreads(int cells)
+{
+    return Pol::kPairs ? std::min(32 * kPairMaxWarps, cells * kPairWidest) : std::min(32 * kMaxWarps, cells);
+}
 
-// Threads per CTA of the pair loop: the block size asked for, doubled up to
-// 512 while the CTAs of the tiles with particles would all be resident at
+// Threads per CTA of a full substep: the block size asked for, doubled up to
+// widest while the CTAs of the tiles with particles would all be resident at
 // once. A launch of few tiles lasts as long as its slowest tile, whose
 // warps' groups then run side by side (and, with more warps than groups, the
-// pairs of rounds of a group). memo keeps the last answer of a caller.
-static int pair_threads(int device, int cells, const void *kernel, const void *wide, size_t (*dyn_bytes)(int),
-                        int threads, int nbusy, PairThreads &memo, int &out)
+// pairs of rounds of a group). FP64, 100,000 particles in about 100 tiles:
+// 128 threads 30.1 us a substep, 256 25.2; 1,000,000 in 1024 tiles: 128
+// threads 72.5, 256 (one CTA per SM) 106. memo keeps the last answer of a caller.
+static int widened_threads(int device, int cells, const void *kernel, const void *wide, size_t (*dyn_bytes)(int),
+                           int threads, int widest, int nbusy, WideThreads &memo, int &out)
 {
     out = threads;
-    if (memo.threads == threads && memo.nbusy == nbusy && memo.cells == cells) {
+    if (memo.kernel == kernel && memo.threads == threads && memo.nbusy == nbusy && memo.cells == cells) {
         out = memo.answer;
         return ICM_OK;
     }
@@ -540,17 +551,20 @@ static int pair_threads(int device, int cells, const void *kernel, const void *w
     ICM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     ICM_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
     // a power of two of warps shares the groups of every tile evenly
-    while ((out & (out - 1)) == 0 && out * 2 <= 32 * kPairMaxWarps && out * 2 <= cells * kPairWidest) {
+    while ((out & (out - 1)) == 0 && out * 2 <= widest) {
+        const void *k = pair_wide(cells, 2 * out) ? wide : kernel;
         const size_t dyn = dyn_bytes(2 * out / 32);
         int per_sm = 0;
-        if (dyn + kPairStaticBytes > (size_t)most) break;
-        const void *k = pair_wide(cells, 2 * out) ? wide : kernel;
+        cudaFuncAttributes fa;
+        ICM_CUDA(cudaFuncGetAttributes(&fa, k));
+        if (dyn + fa.sharedSizeBytes > (size_t)most) break;
         // (all there is: a smaller value would take back what a launch opted in to)
-        ICM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)kPairStaticBytes));
+        ICM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes));
         ICM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 2 * out, dyn));
         if (nbusy > per_sm * sms) break;
         out *= 2;
     }
+    memo.kernel = kernel;
     memo.threads = threads;
     memo.nbusy = nbusy;
     memo.cells = cells;
@@ -567,13 +581,15 @@ static int launch_one(icm_ctx *c, int ntiles, const icy_SimParams &P, const type
     int threads = c->threads;
     if (TX * TY > 32 * kMaxGroupsPerWarp * (threads / 32) || threads / 32 > kMaxWarps)
         return icm::fail(ICM_ERR_ARG, "tile too large for the block size (need threads >= TX*TY/4)");
-    if constexpr (kPairLaunch<Pol, MODE>) {
-        const int rc = pair_threads(c->device, TX * TY, (const void *)k_tile_substep<Pol, TX, TY, kModeFull>,
-                                    (const void *)k_tile_substep<Pol, TX, TY, kModeFullWide>,
-                                    launch_dyn_bytes<Pol, TX, TY, MODE>, c->threads, c->nbusy, c->wide, threads);
+    if constexpr (kWidens<Pol, MODE>) {
+        constexpr int kWideMode = Pol::kPairs ? kModeFullWide : kModeFull;
+        const int rc = widened_threads(c->device, TX * TY, (const void *)k_tile_substep<Pol, TX, TY, kModeFull>,
+                                       (const void *)k_tile_substep<Pol, TX, TY, kWideMode>,
+                                       launch_dyn_bytes<Pol, TX, TY, MODE>, c->threads, kWidestThreads<Pol>(TX * TY),
+                                       c->nbusy, c->wide, threads);
         if (rc) return rc;
-        if constexpr (MODE == kModeFull)
-            if (pair_wide(TX * TY, threads)) return launch_one<Pol, TX, TY, kModeFullWide>(c, ntiles, P, K, A, R);
+        if constexpr (MODE != kWideMode)
+            if (pair_wide(TX * TY, threads)) return launch_one<Pol, TX, TY, kWideMode>(c, ntiles, P, K, A, R);
     }
     const size_t dyn = launch_dyn_bytes<Pol, TX, TY, MODE>(threads / 32);
     static size_t opted[kMaxDevices] = {};  // static + dynamic shared memory above 48 KB needs the opt-in
@@ -1427,7 +1443,7 @@ struct icm_ensemble {
     size_t tiles_cap = 0;
     int nactive = 0;
     int nbusy = 0;     // launch list entries of tiles with particles
-    PairThreads wide;  // threads of the launches (pair_threads)
+    WideThreads wide;  // threads of the launches (widened_threads)
     double *d_ind_x = nullptr;
     size_t ind_x_cap = 0;
     uint8_t *d_active = nullptr;  // every case's tile mask, concatenated
@@ -1468,13 +1484,15 @@ int ens_launch_one(icm_ensemble *e, int grid, const void *d_cases, const EnsLaun
     // its dependency wait: they are ordinary stream-ordered launches
     const bool pdl = (MODE == kModeFull || MODE == kModeFullWide) && L.j > 0;
     int threads = e->threads;
-    if constexpr (kPairLaunch<Pol, MODE>) {
-        const int rc = pair_threads(e->device, TX * TY, (const void *)k_tile_substep_ens<Pol, TX, TY, kModeFull>,
-                                    (const void *)k_tile_substep_ens<Pol, TX, TY, kModeFullWide>,
-                                    launch_dyn_bytes<Pol, TX, TY, MODE>, e->threads, e->nbusy, e->wide, threads);
+    if constexpr (kWidens<Pol, MODE>) {
+        constexpr int kWideMode = Pol::kPairs ? kModeFullWide : kModeFull;
+        const int rc = widened_threads(e->device, TX * TY, (const void *)k_tile_substep_ens<Pol, TX, TY, kModeFull>,
+                                       (const void *)k_tile_substep_ens<Pol, TX, TY, kWideMode>,
+                                       launch_dyn_bytes<Pol, TX, TY, MODE>, e->threads, kWidestThreads<Pol>(TX * TY),
+                                       e->nbusy, e->wide, threads);
         if (rc) return rc;
-        if constexpr (MODE == kModeFull)
-            if (pair_wide(TX * TY, threads)) return ens_launch_one<Pol, TX, TY, kModeFullWide>(e, grid, d_cases, L);
+        if constexpr (MODE != kWideMode)
+            if (pair_wide(TX * TY, threads)) return ens_launch_one<Pol, TX, TY, kWideMode>(e, grid, d_cases, L);
     }
     const size_t dyn = launch_dyn_bytes<Pol, TX, TY, MODE>(threads / 32);
     static size_t opted[kMaxDevices] = {};
