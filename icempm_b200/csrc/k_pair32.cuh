@@ -211,89 +211,91 @@ static __device__ __noinline__ Deferred pair_deferred(const icy_SimParams &P, co
     return d;
 }
 
-struct PairNode { float v0, v1; double f0, f1; int bin; };
-
-// What a CTA at the indenter keeps of its contact nodes until the particle
-// loop starts: the force bins and their total, and the nodes of the region
-// inside the indenter with their velocities.
-__host__ __device__ constexpr size_t pair_contact_bytes(int RN) { return kBinsBytes + 16 + (size_t)RN * (sizeof(float2) + sizeof(int)); }
+// What a CTA at the indenter keeps of the region's nodes inside it until the
+// particle loop starts: a bit per node, and the list of them with their
+// normals and force bins.
+__host__ __device__ constexpr int pair_mask_words(int RN) { return (RN + 31) / 32; }
+__host__ __device__ constexpr size_t pair_contact_bytes(int RN)
+{
+    return (((size_t)4 * (1 + pair_mask_words(RN)) + 15) & ~(size_t)15) + (size_t)RN * (sizeof(double2) + sizeof(int));
+}
 struct PairContact {
-    double *bins, *tot;
-    int *n, *node;
-    float2 *v;
-    __device__ PairContact(double *p, int RN)
-        : bins(p), tot(p + 2 * kMaxBins), n((int *)(p + 2 * kMaxBins + 2)), node((int *)(p + 2 * kMaxBins + 4) + 2 * RN),
-          v((float2 *)(p + 2 * kMaxBins + 4))
+    int *n;           // listed nodes
+    unsigned *mask;   // bit k: node k of the region is listed
+    double2 *normal;
+    int *code;        // node | bin << 16
+    __device__ PairContact(void *p, int RN)
+        : n((int *)p), mask((unsigned *)p + 1),
+          normal((double2 *)((char *)p + pair_contact_bytes(RN)) - RN - RN / 4), code((int *)(normal + RN))
     {
     }
 };
 
-// The region's nodes inside the indenter, listed and dealt out to the
-// threads: a node's contact in FP64 takes about 2,000 cycles, and four nodes
-// in turn per thread were the longest part of a tile at the indenter (8,000
-// cycles, now 3,000). Their velocities wait in the list while every thread
-// updates its nodes as if there were no indenter. (Out of line.)
+// The region's nodes inside the indenter, their normals and bins: known from
+// the indenter's place alone, so listed before the wait for the previous
+// substep. (A node's contact in FP64 takes about 2,000 cycles, most of them
+// in the normal and the angle; after the wait, with the force bins summed in
+// shared memory and two more barriers, contact took 7,500 of the 26,000
+// cycles of a tile at the indenter, the longest of a substep of few tiles.
+// 14,000 particles 16.8 us, now 12.8; 70,000 17.5, now 14.2; 1,000,000 34.6, now
+// 32.2.) (Out of line.)
 template <int TX, int TY>
-static __device__ __noinline__ void pair_contact_begin(const icy_SimParams &P, const Consts32 &K, const TileRun &R,
-                                                       const int x0, const int y0, const bool count, const bool staged,
-                                                       const float4 *s_v, const PairContact C)
+static __device__ __noinline__ void pair_contact_list(const icy_SimParams &P, const TileRun &R, const int x0, const int y0,
+                                                      const PairContact C)
 {
     constexpr int RX = TX + 4, RY = TY + 4, RN = RX * RY;
-    const int tid = threadIdx.x, nthr = blockDim.x, rx0 = x0 - 1, ry0 = y0 - 1;
+    for (int k = threadIdx.x; k < RN; k += blockDim.x) {
+        double n0, n1;
+        if (!contact_normal(P, x0 - 1 + k % RX, y0 - 1 + k / RX, R.ind_x, R.ind_y, n0, n1)) continue;
+        const int e = atomicAdd(C.n, 1);
+        C.normal[e] = make_double2(n0, n1);
+        C.code[e] = k | contact_bin(P, n0, n1) << 16;
+        atomicOr(&C.mask[k >> 5], 1u << (k & 31));
+    }
+}
+
+// The listed nodes' velocities, in place, and the reaction of those that the
+// tile owns (count) to the force bins: as Pol32::node_velocity. The last
+// threads take them, which have the fewest of the region's other nodes.
+template <int TX, int TY>
+static __device__ __noinline__ void pair_contact_nodes(const icy_SimParams &P, const Consts32 &K, const TileRun &R,
+                                                       const int x0, const int y0, const bool count, const bool staged,
+                                                       float4 *s_v, const PairContact C)
+{
+    constexpr int RX = TX + 4;
+    const int nthr = blockDim.x, n = *C.n;
     const float4 *gA = (const float4 *)R.gA;
-    auto node = [&](int k) {
-        const int x = rx0 + k % RX, y = ry0 + k / RX;
-        if (staged) return s_v[k];
-        return x >= 0 && y >= 0 && x < P.GridX && y < P.GridY ? gA[(size_t)y * P.GridX + x] : make_float4(0.f, 0.f, 0.f, 0.f);
-    };
-    for (int k = tid; k < RN; k += nthr) {
-        const double n0 = (rx0 + k % RX) * P.cellsize - R.ind_x, n1 = (ry0 + k / RX) * P.cellsize - R.ind_y;
-        if (n0 * n0 + n1 * n1 < P.IndRSq && node(k).x != 0.0f) C.node[atomicAdd(C.n, 1)] = k;
-    }
-    __syncthreads();
     double tot0 = 0.0, tot1 = 0.0;
-    for (int e = tid; e < *C.n; e += nthr) {
-        const int k = C.node[e], x = rx0 + k % RX, y = ry0 + k / RX;
-        PairNode o{0.f, 0.f, 0.0, 0.0, -1};
-        Pol32::node_velocity(P, K, node(k), x, y, R.ind_x, R.ind_y, o.v0, o.v1, o.f0, o.f1, o.bin, true);
-        C.v[e] = make_float2(o.v0, o.v1);
-        if (o.bin >= 0 && count && x >= x0 && x < x0 + TX && y >= y0 && y < y0 + TY) {
-            atomicAdd(&C.bins[2 * o.bin], o.f0);
-            atomicAdd(&C.bins[2 * o.bin + 1], o.f1);
-            tot0 += o.f0;
-            tot1 += o.f1;
+    for (int e = nthr - 1 - (int)threadIdx.x; e < n; e += nthr) {
+        const int k = C.code[e] & 0xffff, bin = C.code[e] >> 16, x = x0 - 1 + k % RX, y = y0 - 1 + k / RX;
+        const double2 nrm = C.normal[e];
+        float4 nd = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (staged) nd = s_v[k];
+        else if (x >= 0 && y >= 0 && x < P.GridX && y < P.GridY) nd = gA[(size_t)y * P.GridX + x];
+        float a = 0.f, b = 0.f;
+        if (nd.x != 0.0f) {
+            double f0, f1;
+            Pol32::free_velocity(K, nd, a, b);
+            if (contact_slip(P, nd.x, nrm.x, nrm.y, a, b, f0, f1) && count && x >= x0 && x < x0 + TX && y >= y0 && y < y0 + TY) {
+                atomicAdd(&R.bins[2 * bin], f0);
+                atomicAdd(&R.bins[2 * bin + 1], f1);
+                tot0 += f0;
+                tot1 += f1;
+            }
+            Pol32::wall_velocity(P, x, y, a, b);
         }
+        s_v[k] = make_float4(a, a, b, b);
     }
+    if (!R.force_slot || !__any_sync(0xffffffffu, tot0 != 0.0 || tot1 != 0.0)) return;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         tot0 += __shfl_xor_sync(0xffffffffu, tot0, o);
         tot1 += __shfl_xor_sync(0xffffffffu, tot1, o);
     }
-    if ((tid & 31) == 0 && (tot0 != 0.0 || tot1 != 0.0)) {
-        atomicAdd(&C.tot[0], tot0);
-        atomicAdd(&C.tot[1], tot1);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&R.force_slot[0], tot0);
+        atomicAdd(&R.force_slot[1], tot1);
     }
-    __syncthreads();  // every listed node is read before the region is updated in place
-}
-
-// After the update: the listed velocities into the region, the reaction to
-// the force bins.
-template <int TX, int TY>
-static __device__ __noinline__ void pair_contact_end(const icy_SimParams &P, const TileRun &R, float4 *s_v,
-                                                     const PairContact C)
-{
-    const int tid = threadIdx.x, nthr = blockDim.x;
-    for (int e = tid; e < *C.n; e += nthr) {
-        const float2 v = C.v[e];
-        s_v[C.node[e]] = make_float4(v.x, v.x, v.y, v.y);
-    }
-    for (int k = tid; k < 2 * P.n_indenter_subdivisions; k += nthr)
-        if (C.bins[k] != 0.0) atomicAdd(&R.bins[k], C.bins[k]);
-    if (tid == 0 && R.force_slot && (C.tot[0] != 0.0 || C.tot[1] != 0.0)) {
-        atomicAdd(&R.force_slot[0], C.tot[0]);
-        atomicAdd(&R.force_slot[1], C.tot[1]);
-    }
-    __syncthreads();  // the bins' space is staging space from here on
 }
 
 // The node region's copy did not complete within the poll limit: the thread
@@ -318,8 +320,8 @@ constexpr int kPairWidest = 2;
 // Dynamic shared memory of a CTA: the node region (as the tensor copy
 // delivers it, then in place the velocities as {vx, vx, vy, vy}, so that one
 // load gives both halves), the warps' P2G regions, and two staging buffers
-// per warp. The second staging buffers hold the force bins and the list of
-// contact nodes until the particle loop starts.
+// per warp. The second staging buffers hold the list of contact nodes until
+// the particle loop starts.
 __host__ __device__ constexpr size_t pair_dyn_bytes(int RN, int nwarps)
 {
     const size_t stage = (size_t)nwarps * sizeof(Pol32::PairStage), bins = pair_contact_bytes(RN);
@@ -416,7 +418,7 @@ __device__ __forceinline__ void pair_tile_body(const icy_SimParams &P, const Con
     float4 *s_v = reinterpret_cast<float4 *>(s_dyn);
     float4 *s_acc = s_v + RN, *wacc = s_acc + warp * RN;
     Pol32::PairStage *s_stage = reinterpret_cast<Pol32::PairStage *>(s_acc + nwarps * RN);
-    PairContact s_con(reinterpret_cast<double *>(s_stage + nwarps), RN);
+    const PairContact s_con(s_stage + nwarps, RN);
     const int tx = t % R.ntx, ty = t / R.ntx;
     const int x0 = tx * TX, y0 = ty * TY, rx0 = x0 - 1, ry0 = y0 - 1;
     const int GX = P.GridX, GY = P.GridY;
@@ -477,9 +479,10 @@ __device__ __forceinline__ void pair_tile_body(const icy_SimParams &P, const Con
         tc05::mbar_init(&s_tma_bar, 1);
     }
     if (tid == 0) s_any = 0;
-    if (contact) {
-        for (int k = tid; k < 2 * P.n_indenter_subdivisions; k += nthr) s_con.bins[k] = 0.0;
-        if (tid == 0) { s_con.tot[0] = 0.0; s_con.tot[1] = 0.0; *s_con.n = 0; }
+    if (contact && busy) {
+        for (int k = tid; k < 1 + pair_mask_words(RN); k += nthr) s_con.n[k] = 0;  // the mask behind it
+        __syncthreads();
+        pair_contact_list<TX, TY>(P, R, x0, y0, s_con);
     }
     __syncthreads();
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -516,7 +519,7 @@ __device__ __forceinline__ void pair_tile_body(const icy_SimParams &P, const Con
     // thread and pass, so that their loads and divisions overlap.
     bool staged = staging && tc05::mbar_wait(&s_tma_bar, 0, kTmaPolls);
     if (staging && !staged) pair_copy_late(&s_tma_bar, R.err);
-    if (contact) pair_contact_begin<TX, TY>(P, K, R, x0, y0, part != 2, staged, s_v, s_con);
+    if (contact) pair_contact_nodes<TX, TY>(P, K, R, x0, y0, part != 2, staged, s_v, s_con);
     {
         const float4 *gA = (const float4 *)R.gA;
         const bool edge = rx0 <= 2 || ry0 <= 2 || rx0 + RX > GX - 3 || ry0 + RY > GY - 3;
@@ -566,12 +569,14 @@ __device__ __forceinline__ void pair_tile_body(const icy_SimParams &P, const Con
                 }
             }
 #pragma unroll
-            for (int b = 0; b < NB; b++)
-                if (k0 + b * nthr < RN) s_v[k0 + b * nthr] = make_float4(va[b], va[b], vb[b], vb[b]);
+            for (int b = 0; b < NB; b++) {
+                const int k = k0 + b * nthr;
+                if (k >= RN || (contact && (s_con.mask[k >> 5] >> (k & 31) & 1))) continue;
+                s_v[k] = make_float4(va[b], va[b], vb[b], vb[b]);
+            }
         }
     }
     __syncthreads();
-    if (contact) pair_contact_end<TX, TY>(P, R, s_v, s_con);
 
     // the particles of the warp's groups
     int stage = 0;

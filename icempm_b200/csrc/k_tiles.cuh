@@ -501,6 +501,41 @@ static __device__ __noinline__ void harvest_state(const Consts32 &k, const M2f H
 // FP32 strain form: position = int16 cell + 32-bit fixed-point fraction,
 // H = Fe - I, Jp = Jp_inv - 1; meta holds the grain's residues and the
 // crushed flag (grain_meta32). The arithmetic is FP32.
+// FP32 contact, its geometry and reaction in FP64: whether node (gx, gy) is
+// inside the indenter, with the unit vector from its axis,
+__device__ __forceinline__ bool contact_normal(const icy_SimParams &P, int gx, int gy, double ind_x, double ind_y,
+                                               double &n0, double &n1)
+{
+    n0 = gx * P.cellsize - ind_x;
+    n1 = gy * P.cellsize - ind_y;
+    const double z = n0 * n0 + n1 * n1;
+    if (!(z < P.IndRSq)) return false;
+    if (z > 0) { const double nn = sqrt(z); n0 /= nn; n1 /= nn; }
+    return true;
+}
+// the force bin of that direction,
+__device__ __forceinline__ int contact_bin(const icy_SimParams &P, double n0, double n1)
+{
+    double angle = atan2(n0, n1) + ICM_PI;
+    angle *= P.n_indenter_subdivisions / (2 * ICM_PI);
+    return min(max((int)angle, 0), P.n_indenter_subdivisions - 1);
+}
+// and the velocity (a, b) without the part into the indenter, with the
+// reaction; false where the node moves away from it.
+__device__ __forceinline__ bool contact_slip(const icy_SimParams &P, float mass, double n0, double n1, float &a, float &b,
+                                             double &f0, double &f1)
+{
+    const double vco0 = P.IndVelocity, va = a, vb = b, vr0 = va - vco0, vr1 = vb;
+    const double vn = vr0 * n0 + vr1 * n1;
+    if (!(vn < 0)) return false;
+    const double w0 = vco0 + (vr0 - n0 * vn), w1 = vr1 - n1 * vn;
+    f0 = (va - w0) * (double)mass / P.InitialTimeStep;
+    f1 = (vb - w1) * (double)mass / P.InitialTimeStep;
+    a = (float)w0;
+    b = (float)w1;
+    return true;
+}
+
 struct Pol32 {
     static constexpr bool kSurrogate = false;
     static constexpr bool kHarvest = true;
@@ -600,14 +635,12 @@ struct Pol32 {
         return r;
     }
     static __device__ __forceinline__ St load(const Parts &A, int p) { return unpack(A.X[p], A.H[p], A.Jp[p]); }
-    static __device__ __forceinline__ void node_velocity(const icy_SimParams &P, const Consts &k, const Node &n, int gx,
-                                                         int gy, double ind_x, double ind_y, float &v0, float &v1,
-                                                         double &f0, double &f1, int &bin, bool contact)
+    // velocity of a node with mass before contact and walls, and the walls
+    static __device__ __forceinline__ void free_velocity(const Consts &k, const Node &n, float &a, float &b)
     {
-        bin = -1;
-        if (n.x == 0.0f) { v0 = 0.0f; v1 = 0.0f; return; }
         float inv_m = 1.0f / n.x;
-        float a = n.y * inv_m, b = n.z * inv_m;
+        a = n.y * inv_m;
+        b = n.z * inv_m;
         b -= k.dt_g;
         float n2 = a * a + b * b;
         if (n2 > k.vmax * k.vmax) {
@@ -615,38 +648,30 @@ struct Pol32 {
             a *= sc;
             b *= sc;
         }
-        // contact geometry and reaction in FP64, only where the CTA's region
-        // can reach the cylinder
-        if (contact) {
-            double n0 = gx * P.cellsize - ind_x, n1 = gy * P.cellsize - ind_y;
-            if (n0 * n0 + n1 * n1 < P.IndRSq) {
-                const double vco0 = P.IndVelocity;
-                double va = a, vb = b;
-                double vr0 = va - vco0, vr1 = vb;
-                double z = n0 * n0 + n1 * n1;
-                if (z > 0) { double nn = sqrt(z); n0 /= nn; n1 /= nn; }
-                double vn = vr0 * n0 + vr1 * n1;
-                if (vn < 0) {
-                    double vt0 = vr0 - n0 * vn, vt1 = vr1 - n1 * vn;
-                    double w0 = vco0 + vt0, w1 = vt1;
-                    double mass = n.x;
-                    f0 = (va - w0) * mass / P.InitialTimeStep;
-                    f1 = (vb - w1) * mass / P.InitialTimeStep;
-                    double angle = atan2(n0, n1) + ICM_PI;
-                    angle *= P.n_indenter_subdivisions / (2 * ICM_PI);
-                    int index = (int)angle;
-                    index = max(index, 0);
-                    index = min(index, P.n_indenter_subdivisions - 1);
-                    bin = index;
-                    a = (float)w0;
-                    b = (float)w1;
-                }
-            }
-        }
+    }
+    static __device__ __forceinline__ void wall_velocity(const icy_SimParams &P, int gx, int gy, float &a, float &b)
+    {
         if (gy <= 2) { a = 0.0f; b = 0.0f; }
         else if (gy >= P.GridY - 3 && b > 0.0f) b = 0.0f;
         if (gx <= 2 && a < 0.0f) a = 0.0f;
         else if (gx >= P.GridX - 3 && a > 0.0f) a = 0.0f;
+    }
+    static __device__ __forceinline__ void node_velocity(const icy_SimParams &P, const Consts &k, const Node &n, int gx,
+                                                         int gy, double ind_x, double ind_y, float &v0, float &v1,
+                                                         double &f0, double &f1, int &bin, bool contact)
+    {
+        bin = -1;
+        if (n.x == 0.0f) { v0 = 0.0f; v1 = 0.0f; return; }
+        float a, b;
+        free_velocity(k, n, a, b);
+        // contact geometry and reaction in FP64, only where the CTA's region
+        // can reach the cylinder
+        if (contact) {
+            double n0, n1;
+            if (contact_normal(P, gx, gy, ind_x, ind_y, n0, n1) && contact_slip(P, n.x, n0, n1, a, b, f0, f1))
+                bin = contact_bin(P, n0, n1);
+        }
+        wall_velocity(P, gx, gy, a, b);
         v0 = a; v1 = b;
     }
     static __device__ __forceinline__ Tau<float> stress(const icy_SimParams &, const Consts &k, const St &s)
