@@ -211,91 +211,32 @@ static __device__ __noinline__ Deferred pair_deferred(const icy_SimParams &P, co
     return d;
 }
 
-// What a CTA at the indenter keeps of the region's nodes inside it until the
-// particle loop starts: a bit per node, and the list of them with their
-// normals and force bins.
-__host__ __device__ constexpr int pair_mask_words(int RN) { return (RN + 31) / 32; }
-__host__ __device__ constexpr size_t pair_contact_bytes(int RN)
-{
-    return (((size_t)4 * (1 + pair_mask_words(RN)) + 15) & ~(size_t)15) + (size_t)RN * (sizeof(double2) + sizeof(int));
-}
-struct PairContact {
-    int *n;           // listed nodes
-    unsigned *mask;   // bit k: node k of the region is listed
-    double2 *normal;
-    int *code;        // node | bin << 16
-    __device__ PairContact(void *p, int RN)
-        : n((int *)p), mask((unsigned *)p + 1),
-          normal((double2 *)((char *)p + pair_contact_bytes(RN)) - RN - RN / 4), code((int *)(normal + RN))
-    {
-    }
-};
-
-// The region's nodes inside the indenter, their normals and bins: known from
-// the indenter's place alone, so listed before the wait for the previous
-// substep. (A node's contact in FP64 takes about 2,000 cycles, most of them
-// in the normal and the angle; after the wait, with the force bins summed in
-// shared memory and two more barriers, contact took 7,500 of the 26,000
-// cycles of a tile at the indenter, the longest of a substep of few tiles.
-// 14,000 particles 16.8 us, now 12.8; 70,000 17.5, now 14.2; 1,000,000 34.6, now
-// 32.2.) (Out of line.)
-template <int TX, int TY>
-static __device__ __noinline__ void pair_contact_list(const icy_SimParams &P, const TileRun &R, const int x0, const int y0,
-                                                      const PairContact C)
-{
-    constexpr int RX = TX + 4, RY = TY + 4, RN = RX * RY;
-    for (int k = threadIdx.x; k < RN; k += blockDim.x) {
-        double n0, n1;
-        if (!contact_normal(P, x0 - 1 + k % RX, y0 - 1 + k / RX, R.ind_x, R.ind_y, n0, n1)) continue;
-        const int e = atomicAdd(C.n, 1);
-        C.normal[e] = make_double2(n0, n1);
-        C.code[e] = k | contact_bin(P, n0, n1) << 16;
-        atomicOr(&C.mask[k >> 5], 1u << (k & 31));
-    }
-}
-
 // The listed nodes' velocities, in place, and the reaction of those that the
 // tile owns (count) to the force bins: as Pol32::node_velocity. The last
 // threads take them, which have the fewest of the region's other nodes.
 template <int TX, int TY>
 static __device__ __noinline__ void pair_contact_nodes(const icy_SimParams &P, const Consts32 &K, const TileRun &R,
                                                        const int x0, const int y0, const bool count, const bool staged,
-                                                       float4 *s_v, const PairContact C)
+                                                       float4 *s_v, const ContactList C)
 {
     constexpr int RX = TX + 4;
     const int nthr = blockDim.x, n = *C.n;
     const float4 *gA = (const float4 *)R.gA;
-    double tot0 = 0.0, tot1 = 0.0;
+    NodeForce force;
     for (int e = nthr - 1 - (int)threadIdx.x; e < n; e += nthr) {
         const int k = C.code[e] & 0xffff, bin = C.code[e] >> 16, x = x0 - 1 + k % RX, y = y0 - 1 + k / RX;
         const double2 nrm = C.normal[e];
         float4 nd = make_float4(0.f, 0.f, 0.f, 0.f);
         if (staged) nd = s_v[k];
         else if (x >= 0 && y >= 0 && x < P.GridX && y < P.GridY) nd = gA[(size_t)y * P.GridX + x];
-        float a = 0.f, b = 0.f;
-        if (nd.x != 0.0f) {
-            double f0, f1;
-            Pol32::free_velocity(K, nd, a, b);
-            if (contact_slip(P, nd.x, nrm.x, nrm.y, a, b, f0, f1) && count && x >= x0 && x < x0 + TX && y >= y0 && y < y0 + TY) {
-                atomicAdd(&R.bins[2 * bin], f0);
-                atomicAdd(&R.bins[2 * bin + 1], f1);
-                tot0 += f0;
-                tot1 += f1;
-            }
-            Pol32::wall_velocity(P, x, y, a, b);
-        }
+        float a, b;
+        double f0, f1;
+        if (Pol32::contact_velocity(P, K, nd, x, y, nrm.x, nrm.y, a, b, f0, f1) && count && x >= x0 && x < x0 + TX &&
+            y >= y0 && y < y0 + TY)
+            force.add(R, bin, f0, f1);
         s_v[k] = make_float4(a, a, b, b);
     }
-    if (!R.force_slot || !__any_sync(0xffffffffu, tot0 != 0.0 || tot1 != 0.0)) return;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        tot0 += __shfl_xor_sync(0xffffffffu, tot0, o);
-        tot1 += __shfl_xor_sync(0xffffffffu, tot1, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&R.force_slot[0], tot0);
-        atomicAdd(&R.force_slot[1], tot1);
-    }
+    force.total(R);
 }
 
 // The node region's copy did not complete within the poll limit: the thread
@@ -324,7 +265,7 @@ constexpr int kPairWidest = 2;
 // the particle loop starts.
 __host__ __device__ constexpr size_t pair_dyn_bytes(int RN, int nwarps)
 {
-    const size_t stage = (size_t)nwarps * sizeof(Pol32::PairStage), bins = pair_contact_bytes(RN);
+    const size_t stage = (size_t)nwarps * sizeof(Pol32::PairStage), bins = contact_bytes(RN);
     return (size_t)RN * 16 * (1 + nwarps) + stage + (stage > bins ? stage : bins);
 }
 
@@ -418,7 +359,7 @@ __device__ __forceinline__ void pair_tile_body(const icy_SimParams &P, const Con
     float4 *s_v = reinterpret_cast<float4 *>(s_dyn);
     float4 *s_acc = s_v + RN, *wacc = s_acc + warp * RN;
     Pol32::PairStage *s_stage = reinterpret_cast<Pol32::PairStage *>(s_acc + nwarps * RN);
-    const PairContact s_con(s_stage + nwarps, RN);
+    const ContactList s_con(s_stage + nwarps, RN);
     const int tx = t % R.ntx, ty = t / R.ntx;
     const int x0 = tx * TX, y0 = ty * TY, rx0 = x0 - 1, ry0 = y0 - 1;
     const int GX = P.GridX, GY = P.GridY;
@@ -480,9 +421,9 @@ __device__ __forceinline__ void pair_tile_body(const icy_SimParams &P, const Con
     }
     if (tid == 0) s_any = 0;
     if (contact && busy) {
-        for (int k = tid; k < 1 + pair_mask_words(RN); k += nthr) s_con.n[k] = 0;  // the mask behind it
+        for (int k = tid; k < 1 + contact_mask_words(RN); k += nthr) s_con.n[k] = 0;  // the mask behind it
         __syncthreads();
-        pair_contact_list<TX, TY>(P, R, x0, y0, s_con);
+        contact_list<TX, TY>(P, R, x0, y0, s_con);
     }
     __syncthreads();
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -440,8 +440,21 @@ struct Pol64 {
     {
         bin = -1;
         if (n.m == 0) { v0 = 0; v1 = 0; return; }
-        NodeOut o = update_node64(P, gx, gy, n.m, n.px, n.py, contact ? ix : 1e300, iy);
+        NodeOut o = contact ? update_node64(P, gx, gy, n.m, n.px, n.py, ix, iy)
+                            : update_node64<false>(P, gx, gy, n.m, n.px, n.py, ix, iy);
         v0 = o.v0; v1 = o.v1; f0 = o.f0; f1 = o.f1; bin = o.bin;
+    }
+    // of a node inside the indenter, given its normal; whether it is in contact
+    static __device__ __forceinline__ bool contact_velocity(const icy_SimParams &P, const Consts &, const Node &n, int gx,
+                                                            int gy, double n0, double n1, double &v0, double &v1,
+                                                            double &f0, double &f1)
+    {
+        v0 = v1 = 0;
+        if (n.m == 0) return false;
+        free_velocity64(P, n.m, n.px, n.py, v0, v1);
+        const bool slip = contact_slip64(P, n.m, n0, n1, v0, v1, f0, f1);
+        wall_velocity64(P, gx, gy, v0, v1);
+        return slip;
     }
     static __device__ __forceinline__ Tau<double> stress(const icy_SimParams &P, const Consts &, const St &s)
     {
@@ -501,36 +514,12 @@ static __device__ __noinline__ void harvest_state(const Consts32 &k, const M2f H
 // FP32 strain form: position = int16 cell + 32-bit fixed-point fraction,
 // H = Fe - I, Jp = Jp_inv - 1; meta holds the grain's residues and the
 // crushed flag (grain_meta32). The arithmetic is FP32.
-// FP32 contact, its geometry and reaction in FP64: whether node (gx, gy) is
-// inside the indenter, with the unit vector from its axis,
-__device__ __forceinline__ bool contact_normal(const icy_SimParams &P, int gx, int gy, double ind_x, double ind_y,
-                                               double &n0, double &n1)
-{
-    n0 = gx * P.cellsize - ind_x;
-    n1 = gy * P.cellsize - ind_y;
-    const double z = n0 * n0 + n1 * n1;
-    if (!(z < P.IndRSq)) return false;
-    if (z > 0) { const double nn = sqrt(z); n0 /= nn; n1 /= nn; }
-    return true;
-}
-// the force bin of that direction,
-__device__ __forceinline__ int contact_bin(const icy_SimParams &P, double n0, double n1)
-{
-    double angle = atan2(n0, n1) + ICM_PI;
-    angle *= P.n_indenter_subdivisions / (2 * ICM_PI);
-    return min(max((int)angle, 0), P.n_indenter_subdivisions - 1);
-}
-// and the velocity (a, b) without the part into the indenter, with the
-// reaction; false where the node moves away from it.
+// FP32 contact, in FP64 (contact_slip64) from the rounded velocity (a, b)
 __device__ __forceinline__ bool contact_slip(const icy_SimParams &P, float mass, double n0, double n1, float &a, float &b,
                                              double &f0, double &f1)
 {
-    const double vco0 = P.IndVelocity, va = a, vb = b, vr0 = va - vco0, vr1 = vb;
-    const double vn = vr0 * n0 + vr1 * n1;
-    if (!(vn < 0)) return false;
-    const double w0 = vco0 + (vr0 - n0 * vn), w1 = vr1 - n1 * vn;
-    f0 = (va - w0) * (double)mass / P.InitialTimeStep;
-    f1 = (vb - w1) * (double)mass / P.InitialTimeStep;
+    double w0 = a, w1 = b;
+    if (!contact_slip64(P, mass, n0, n1, w0, w1, f0, f1)) return false;
     a = (float)w0;
     b = (float)w1;
     return true;
@@ -673,6 +662,18 @@ struct Pol32 {
         }
         wall_velocity(P, gx, gy, a, b);
         v0 = a; v1 = b;
+    }
+    // of a node inside the indenter, given its normal; whether it is in contact
+    static __device__ __forceinline__ bool contact_velocity(const icy_SimParams &P, const Consts &k, const Node &n, int gx,
+                                                            int gy, double n0, double n1, float &v0, float &v1,
+                                                            double &f0, double &f1)
+    {
+        v0 = v1 = 0.0f;
+        if (n.x == 0.0f) return false;
+        free_velocity(k, n, v0, v1);
+        const bool slip = contact_slip(P, n.x, n0, n1, v0, v1, f0, f1);
+        wall_velocity(P, gx, gy, v0, v1);
+        return slip;
     }
     static __device__ __forceinline__ Tau<float> stress(const icy_SimParams &, const Consts &k, const St &s)
     {
@@ -1130,6 +1131,35 @@ __device__ __forceinline__ int stray_scatter(const icy_SimParams &P, const typen
     return bad;
 }
 
+// The indenter's reaction of a thread's nodes: to its bin node by node, to
+// the run's total once per warp, straight to global memory. (Sums in shared
+// memory took compare-and-swap loops, all nodes of a tile on one total, and
+// two barriers for the flush.)
+struct NodeForce {
+    double f0 = 0.0, f1 = 0.0;
+    __device__ __forceinline__ void add(const TileRun &R, int bin, double a, double b)
+    {
+        atomicAdd(&R.bins[2 * bin], a);
+        atomicAdd(&R.bins[2 * bin + 1], b);
+        f0 += a;
+        f1 += b;
+    }
+    // (by whole warps)
+    __device__ __forceinline__ void total(const TileRun &R)
+    {
+        if (!R.force_slot || !__any_sync(0xffffffffu, f0 != 0.0 || f1 != 0.0)) return;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            f0 += __shfl_xor_sync(0xffffffffu, f0, o);
+            f1 += __shfl_xor_sync(0xffffffffu, f1, o);
+        }
+        if ((threadIdx.x & 31) == 0) {
+            atomicAdd(&R.force_slot[0], f0);
+            atomicAdd(&R.force_slot[1], f1);
+        }
+    }
+};
+
 // Whether a node of tile t's (TX+4) x (TY+4) region lies inside the
 // indenter's circle.
 template <int TX, int TY>
@@ -1143,6 +1173,81 @@ __device__ __forceinline__ bool region_touches_indenter(const icy_SimParams &P, 
     return dx * dx + dy * dy <= r * r;
 }
 
+// What a CTA at the indenter keeps of the region's nodes inside it until the
+// particle loop starts: a bit per node, and the list of them with their
+// normals and force bins.
+__host__ __device__ constexpr int contact_mask_words(int RN) { return (RN + 31) / 32; }
+__host__ __device__ constexpr size_t contact_bytes(int RN)
+{
+    return (((size_t)4 * (1 + contact_mask_words(RN)) + 15) & ~(size_t)15) + (size_t)RN * (sizeof(double2) + sizeof(int));
+}
+struct ContactList {
+    int *n;           // listed nodes
+    unsigned *mask;   // bit k: node k of the region is listed
+    double2 *normal;
+    int *code;        // node | bin << 16
+    __device__ ContactList(void *p, int RN)
+        : n((int *)p), mask((unsigned *)p + 1),
+          normal((double2 *)((char *)p + contact_bytes(RN)) - RN - RN / 4), code((int *)(normal + RN))
+    {
+    }
+};
+
+// The region's nodes inside the indenter, their normals and bins: known from
+// the indenter's place alone, so listed before the wait for the previous
+// substep. (A node's contact in FP64 takes about 2,000 cycles, most of them
+// in the normal and the angle; after the wait, with the force bins summed in
+// shared memory and two more barriers, contact took 7,500 of the 26,000
+// cycles of a tile at the indenter, the longest of a substep of few tiles.
+// 14,000 particles 16.8 us, now 12.8; 70,000 17.5, now 14.2; 1,000,000 34.6, now
+// 32.2.) (Out of line.)
+template <int TX, int TY>
+static __device__ __noinline__ void contact_list(const icy_SimParams &P, const TileRun &R, const int x0, const int y0,
+                                                      const ContactList C)
+{
+    constexpr int RX = TX + 4, RY = TY + 4, RN = RX * RY;
+    for (int k = threadIdx.x; k < RN; k += blockDim.x) {
+        double n0, n1;
+        if (!contact_normal(P, x0 - 1 + k % RX, y0 - 1 + k / RX, R.ind_x, R.ind_y, n0, n1)) continue;
+        const int e = atomicAdd(C.n, 1);
+        C.normal[e] = make_double2(n0, n1);
+        C.code[e] = k | contact_bin(P, n0, n1) << 16;
+        atomicOr(&C.mask[k >> 5], 1u << (k & 31));
+    }
+}
+
+// The listed nodes' velocities and the reaction of those that the tile owns
+// (count) to the force bins; the update of the others leaves them out. (Out
+// of line, with the geometry before the wait: contact inside the update's
+// loop cost every tile registers, and the nodes of one thread in turn made
+// the tiles at the indenter the last to end. FP64, 1,000,000 particles 71.5
+// us a substep, now 67; 100,000 25.2, now 23.5.)
+template <class Pol, int TX, int TY>
+static __device__ __noinline__ void tile_contact(const icy_SimParams &P, const typename Pol::Consts &K, const TileRun &R,
+                                                 const int x0, const int y0, const bool count,
+                                                 const typename Pol::Node *staged, typename Pol::V2 *s_v,
+                                                 const ContactList C)
+{
+    constexpr int RX = TX + 4;
+    const int nthr = blockDim.x, n = *C.n;
+    const typename Pol::Node *gA = (const typename Pol::Node *)R.gA;
+    NodeForce force;
+    for (int e = nthr - 1 - (int)threadIdx.x; e < n; e += nthr) {
+        const int k = C.code[e] & 0xffff, bin = C.code[e] >> 16, x = x0 - 1 + k % RX, y = y0 - 1 + k / RX;
+        const double2 nrm = C.normal[e];
+        typename Pol::real v0 = 0, v1 = 0;
+        double f0, f1;
+        if (x >= 0 && y >= 0 && x < P.GridX && y < P.GridY &&
+            Pol::contact_velocity(P, K, staged ? staged[k] : gA[(size_t)y * P.GridX + x], x, y, nrm.x, nrm.y, v0, v1, f0,
+                                  f1) &&
+            count && x >= x0 && x < x0 + TX && y >= y0 && y < y0 + TY)
+            force.add(R, bin, f0, f1);
+        s_v[k].x = v0;
+        s_v[k].y = v1;
+    }
+    force.total(R);
+}
+
 // Dynamic shared memory of one CTA (host and kernel use the same layout):
 // the warps' P2G regions (none in the final launch), then Pol::kStages
 // staging rounds per warp.
@@ -1151,17 +1256,13 @@ __host__ __device__ constexpr size_t tile_region_bytes(int RN, int nwarps)
 {
     return (MODE == kModeFinal) ? 0 : (size_t)nwarps * RN * sizeof(typename Pol::Acc);
 }
-// The staging rounds share their space with the reduction of the indenter
-// force (2 kMaxBins bins and the total, doubles), which is done with before
-// the first round is staged.
-constexpr size_t kBinsBytes = (2 * kMaxBins + 2) * sizeof(double);
+// The staging rounds share their space with the list of contact nodes, which
+// is done with before the first round is staged.
 template <class Pol, int MODE>
 __host__ __device__ constexpr size_t tile_dyn_bytes(int RN, int nwarps)
 {
-    return tile_region_bytes<Pol, MODE>(RN, nwarps) +
-           ((size_t)nwarps * Pol::kStages * sizeof(typename Pol::Stage) > kBinsBytes
-                ? (size_t)nwarps * Pol::kStages * sizeof(typename Pol::Stage)
-                : kBinsBytes);
+    const size_t stages = (size_t)nwarps * Pol::kStages * sizeof(typename Pol::Stage);
+    return tile_region_bytes<Pol, MODE>(RN, nwarps) + (stages > contact_bytes(RN) ? stages : contact_bytes(RN));
 }
 
 // One substep of one tile (the body of k_tile_substep). Every return is
@@ -1181,7 +1282,7 @@ __device__ __forceinline__ void tile_body(const icy_SimParams &P, const typename
     extern __shared__ __align__(128) unsigned char s_dyn[];
     Acc *s_acc = reinterpret_cast<Acc *>(s_dyn);
     __shared__ uint64_t s_tma_bar;
-    __shared__ int s_contact, s_mark[9];
+    __shared__ int s_mark[9];
     __shared__ typename Pol::Tables s_tab;
     // per lane of each of the warp's groups: its cell inside the tile
     // (bits 16-31) and the cell's particle count (bits 0-15)
@@ -1194,9 +1295,6 @@ __device__ __forceinline__ void tile_body(const icy_SimParams &P, const typename
     const int GX = P.GridX, GY = P.GridY;
     const int p0 = R.tile_start[t], p1 = R.tile_start[t + 1];
     const int tid = threadIdx.x, nthr = blockDim.x;
-    // force bins and total of the tile's contact nodes, in the staging space
-    double *s_bins = reinterpret_cast<double *>(s_dyn + tile_region_bytes<Pol, MODE>(RN, nthr >> 5));
-    double *s_tot = s_bins + 2 * kMaxBins;
     Node *gA = (Node *)R.gA;
     Node *gB = (Node *)R.gB;
     const unsigned FULL = 0xffffffffu;
@@ -1230,6 +1328,16 @@ __device__ __forceinline__ void tile_body(const icy_SimParams &P, const typename
         }
         __syncwarp();
         if (MODE != kModeP2GOnly) Pol::init_tables(s_tab, K, tid, nthr);
+    }
+    // can any node of the region touch the indenter? (listed here where the
+    // tile has particles, and where it runs on for its nodes' reaction alone)
+    const bool contact_possible = MODE != kModeP2GOnly && region_touches_indenter<TX, TY>(P, R, t);
+    const ContactList s_con(s_dyn + tile_region_bytes<Pol, MODE>(RN, nthr >> 5), RN);
+    if (contact_possible) {
+        for (int k = tid; k < 1 + contact_mask_words(RN); k += nthr) s_con.n[k] = 0;  // the mask behind it
+        __syncthreads();
+        contact_list<TX, TY>(P, R, x0, y0, s_con);
+        __syncthreads();
     }
     // a full substep of a tile with particles stages its node region with
     // one tensor copy (below, after the wait); a descriptor in global memory
@@ -1270,16 +1378,6 @@ __device__ __forceinline__ void tile_body(const icy_SimParams &P, const typename
     const int np = p1 - p0;
     if (np == 0 && !has_mass) return;
 
-    // can any node of the region touch the indenter?
-    bool contact_possible = false;
-    if (MODE != kModeP2GOnly) {
-        contact_possible = region_touches_indenter<TX, TY>(P, R, t);
-        if (contact_possible) {
-            for (int k = tid; k < 2 * P.n_indenter_subdivisions; k += nthr) s_bins[k] = 0.0;
-            if (tid == 0) { s_tot[0] = 0.0; s_tot[1] = 0.0; s_contact = 0; }
-            __syncthreads();
-        }
-    }
     if (tid < 9) s_mark[tid] = 0;
 
     // 2. grid update of the region (velocities into shared memory)
@@ -1305,45 +1403,24 @@ __device__ __forceinline__ void tile_body(const icy_SimParams &P, const typename
                 for (int b = 0; b < NB; b++) {
                     const int k = k0 + b * nthr;
                     if (k >= RN) break;
+                    if (contact_possible && (s_con.mask[k >> 5] >> (k & 31) & 1)) continue;
                     const int gx = rx0 + k % RX, gy = ry0 + k / RX;
                     real v0 = 0, v1 = 0;
                     if (gx >= 0 && gy >= 0 && gx < GX && gy < GY) {
-                        double f0 = 0, f1 = 0;
+                        double f0, f1;
                         int bin;
-                        Pol::node_velocity(P, K, nd[b], gx, gy, R.ind_x, R.ind_y, v0, v1, f0, f1, bin, contact_possible);
-                        bool own = part != 2 && gx >= x0 && gx < x0 + TX && gy >= y0 && gy < y0 + TY;
-                        if (bin >= 0 && own) {
-                            atomicAdd(&s_bins[2 * bin], f0);
-                            atomicAdd(&s_bins[2 * bin + 1], f1);
-                            atomicAdd(&s_tot[0], f0);
-                            atomicAdd(&s_tot[1], f1);
-                            s_contact = 1;
-                        }
+                        Pol::node_velocity(P, K, nd[b], gx, gy, R.ind_x, R.ind_y, v0, v1, f0, f1, bin, false);
                     }
                     s_v[k].x = v0;
                     s_v[k].y = v1;
                 }
             }
+            if (contact_possible)
+                tile_contact<Pol, TX, TY>(P, K, R, x0, y0, part != 2, staged ? s_nodes : nullptr, s_v, s_con);
         } else if (contact_possible && part != 2) {
             // no particles here: only the reaction of this tile's own nodes
             // (counted once, by the first half when the tile runs split)
-            for (int k = tid; k < TX * TY; k += nthr) {
-                const int gx = x0 + k % TX, gy = y0 + k / TX;
-                if (gx < GX && gy < GY) {
-                    Node n = gA[(size_t)gy * GX + gx];
-                    real v0, v1;
-                    double f0 = 0, f1 = 0;
-                    int bin;
-                    Pol::node_velocity(P, K, n, gx, gy, R.ind_x, R.ind_y, v0, v1, f0, f1, bin, true);
-                    if (bin >= 0) {
-                        atomicAdd(&s_bins[2 * bin], f0);
-                        atomicAdd(&s_bins[2 * bin + 1], f1);
-                        atomicAdd(&s_tot[0], f0);
-                        atomicAdd(&s_tot[1], f1);
-                        s_contact = 1;
-                    }
-                }
-            }
+            tile_contact<Pol, TX, TY>(P, K, R, x0, y0, true, nullptr, s_v, s_con);
         }
     }
     const int nwarps_blk = nthr >> 5;
@@ -1351,15 +1428,6 @@ __device__ __forceinline__ void tile_body(const icy_SimParams &P, const typename
     if (MODE != kModeFinal)
         for (int k = tid; k < RN * nwarps_blk; k += nthr) acc_zero(s_acc[k]);
     __syncthreads();
-    if (MODE != kModeP2GOnly && contact_possible && s_contact) {
-        for (int k = tid; k < 2 * P.n_indenter_subdivisions; k += nthr)
-            if (s_bins[k] != 0.0) atomicAdd(&R.bins[k], s_bins[k]);
-        if (tid == 0 && R.force_slot) {
-            atomicAdd(&R.force_slot[0], s_tot[0]);
-            atomicAdd(&R.force_slot[1], s_tot[1]);
-        }
-        __syncthreads();  // the bins' space is staging space from here on
-    }
     if (np == 0) return;
 
     // 3.-4. particles, one lane per grid cell. A lane walks the particles

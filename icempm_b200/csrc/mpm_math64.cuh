@@ -285,54 +285,68 @@ __device__ __forceinline__ Stencil64 stencil64(double x, double y, double h_inv)
 }
 
 // Grid-node velocity update of v2_kernel_update_nodes
-// (gpu_implementation5.cu:221-289) for a node with mass > 0. Returns the
-// reaction force on the indenter in f0/f1 and the angular bin (or -1).
-struct NodeOut { double v0, v1, f0, f1; int bin; };
-
-__device__ __forceinline__ NodeOut update_node64(const icy_SimParams &P, int ix, int iy, double mass,
-                                                 double p0, double p1, double ind_x, double ind_y)
+// (gpu_implementation5.cu:221-289) for a node with mass > 0, in three parts:
+// the velocity before contact and walls,
+__device__ __forceinline__ void free_velocity64(const icy_SimParams &P, double mass, double p0, double p1, double &v0,
+                                                double &v1)
 {
-    const double dt = P.InitialTimeStep, cellsize = P.cellsize;
-    NodeOut o;
-    o.f0 = 0;
-    o.f1 = 0;
-    o.bin = -1;
-    double v0 = p0 / mass, v1 = p1 / mass;
+    const double dt = P.InitialTimeStep;
+    v0 = p0 / mass;
+    v1 = p1 / mass;
     v1 -= dt * P.Gravity;
-    double vmax = 0.5 * cellsize / dt;
+    double vmax = 0.5 * P.cellsize / dt;
     double nrm = sqrt(v0 * v0 + v1 * v1);
     if (nrm > vmax) {
         v0 = v0 / nrm * vmax;
         v1 = v1 / nrm * vmax;
     }
-    double n0 = ix * cellsize - ind_x;
-    double n1 = iy * cellsize - ind_y;
-    if (n0 * n0 + n1 * n1 < P.IndRSq) {
-        const double vco0 = P.IndVelocity, vco1 = 0;
-        double vr0 = v0 - vco0, vr1 = v1 - vco1;
-        double z = n0 * n0 + n1 * n1;
-        if (z > 0) {
-            double nn = sqrt(z);
-            n0 /= nn;
-            n1 /= nn;
-        }
-        double vn = vr0 * n0 + vr1 * n1;
-        if (vn < 0) {
-            double vt0 = vr0 - n0 * vn, vt1 = vr1 - n1 * vn;
-            double pv0 = v0, pv1 = v1;
-            v0 = vco0 + vt0;
-            v1 = vco1 + vt1;
-            o.f0 = (pv0 - v0) * mass / dt;
-            o.f1 = (pv1 - v1) * mass / dt;
-            double angle = atan2(n0, n1);
-            angle += ICM_PI;
-            angle *= P.n_indenter_subdivisions / (2 * ICM_PI);
-            int index = (int)angle;
-            index = max(index, 0);
-            index = min(index, P.n_indenter_subdivisions - 1);
-            o.bin = index;
-        }
+}
+
+// contact: whether node (gx, gy) is inside the indenter, with the unit vector
+// from its axis,
+__device__ __forceinline__ bool contact_normal(const icy_SimParams &P, int gx, int gy, double ind_x, double ind_y,
+                                               double &n0, double &n1)
+{
+    n0 = gx * P.cellsize - ind_x;
+    n1 = gy * P.cellsize - ind_y;
+    const double z = n0 * n0 + n1 * n1;
+    if (!(z < P.IndRSq)) return false;
+    if (z > 0) {
+        const double nn = sqrt(z);
+        n0 /= nn;
+        n1 /= nn;
     }
+    return true;
+}
+// the angular force bin of that direction,
+__device__ __forceinline__ int contact_bin(const icy_SimParams &P, double n0, double n1)
+{
+    double angle = atan2(n0, n1);
+    angle += ICM_PI;
+    angle *= P.n_indenter_subdivisions / (2 * ICM_PI);
+    return min(max((int)angle, 0), P.n_indenter_subdivisions - 1);
+}
+// and the velocity without its part into the indenter, with the reaction
+// (false, and neither, where the node moves away from it),
+__device__ __forceinline__ bool contact_slip64(const icy_SimParams &P, double mass, double n0, double n1, double &v0,
+                                               double &v1, double &f0, double &f1)
+{
+    const double vco0 = P.IndVelocity, vco1 = 0;
+    double vr0 = v0 - vco0, vr1 = v1 - vco1;
+    double vn = vr0 * n0 + vr1 * n1;
+    if (!(vn < 0)) return false;
+    double vt0 = vr0 - n0 * vn, vt1 = vr1 - n1 * vn;
+    double pv0 = v0, pv1 = v1;
+    v0 = vco0 + vt0;
+    v1 = vco1 + vt1;
+    f0 = (pv0 - v0) * mass / P.InitialTimeStep;
+    f1 = (pv1 - v1) * mass / P.InitialTimeStep;
+    return true;
+}
+
+// and the grid's walls.
+__device__ __forceinline__ void wall_velocity64(const icy_SimParams &P, int ix, int iy, double &v0, double &v1)
+{
     if (iy <= 2) {
         v0 = 0;
         v1 = 0;
@@ -343,8 +357,28 @@ __device__ __forceinline__ NodeOut update_node64(const icy_SimParams &P, int ix,
         v0 = 0;
     else if (ix >= P.GridX - 3 && v0 > 0)
         v0 = 0;
-    o.v0 = v0;
-    o.v1 = v1;
+}
+
+// All three. Returns the reaction force on the indenter in f0/f1 and the
+// angular bin (or -1). Without CONTACT the node is known to lie outside the
+// indenter.
+struct NodeOut { double v0, v1, f0, f1; int bin; };
+
+template <bool CONTACT = true>
+__device__ __forceinline__ NodeOut update_node64(const icy_SimParams &P, int ix, int iy, double mass,
+                                                 double p0, double p1, double ind_x, double ind_y)
+{
+    NodeOut o;
+    o.f0 = 0;
+    o.f1 = 0;
+    o.bin = -1;
+    free_velocity64(P, mass, p0, p1, o.v0, o.v1);
+    if (CONTACT) {
+        double n0, n1;
+        if (contact_normal(P, ix, iy, ind_x, ind_y, n0, n1) && contact_slip64(P, mass, n0, n1, o.v0, o.v1, o.f0, o.f1))
+            o.bin = contact_bin(P, n0, n1);
+    }
+    wall_velocity64(P, ix, iy, o.v0, o.v1);
     return o;
 }
 
