@@ -18,20 +18,23 @@
 //   * dirty[b][t] flags tile t of buffer b as possibly non-zero.
 //
 // One CTA owns one node tile t and its particles:
+// (FP32 full substeps: pair_tile_body in k_pair32.cuh, with the same steps,
+// two particles per lane.)
 //   1. zero t's nodes in G[(s+2)%3] if dirty;
 //   2. grid update (v2_kernel_update_nodes, gpu_implementation5.cu:215-290)
 //      of the (TX+4) x (TY+4) node region around t into shared memory: the
 //      region is every node a particle of t can reach after drifting up to
 //      one node from its tile. Halo nodes are recomputed by neighbouring CTAs
 //      (the update is a pure function of the node); only the owner of a node
-//      adds its reaction force, reduced in shared memory in FP64;
+//      adds its reaction force, in FP64;
 //   3. per particle G2P (v2_kernel_g2p, :294-379) from the shared velocities,
 //      advection, Fe update, constitutive model, store;
 //   4. P2G (v2_kernel_p2g, :148-213) of the updated particle for substep s+1.
 //      Particles are walked cell by cell, one lane per cell, so the P2G sums
 //      of a cell (all its particles share the 3x3 stencil) stay in registers
-//      and reach the warp's shared region in 9 conflict-free steps; particles
-//      whose stencil leaves the region fall back to global atomics;
+//      and reach the warp's shared region in 9 conflict-free steps; a particle
+//      that left its cell is added by the whole warp, node by node, and one
+//      whose stencil leaves the region by global atomics;
 //   5. the warps' shared regions are added to G[(s+1)%3] with one vector
 //      atomic per touched node (red.global.add.v4.f32 in FP32) and the
 //      touched tiles are flagged dirty.

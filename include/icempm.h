@@ -43,7 +43,7 @@ enum {
 
 /* Precision / execution forms of icm_run_substeps. */
 enum {
-    ICM_FORM_FP64_STEPWISE = 0, /* reference structure: reset, P2G, update, G2P launches per substep, FP64 */
+    ICM_FORM_FP64_STEPWISE = 0, /* reference structure: P2G, update, G2P launches per substep, FP64 */
     ICM_FORM_FP64 = 1,          /* fused tile substep, FP64 reference form */
     ICM_FORM_FP32 = 2,          /* fused tile substep, FP32 strain form */
     ICM_FORM_FP32_SURROGATE = 3, /* FP32 form with the learned Drucker-Prager projection (icm_set_surrogate) */
@@ -105,7 +105,9 @@ int icm_set_form(icm_ctx *ctx, int form);
 int icm_get_form(icm_ctx *ctx);
 /* Tile shape of the fused forms: index into the built variants
  * (0: 16x8, 1: 16x16, 2: 32x8, 3: 32x16 nodes) and block size (default
- * 16x16 nodes, 128 threads). */
+ * 16x16 nodes, 128 threads). Full substeps of the FP32 and FP64 forms run
+ * with more threads (up to 512 and 256) while the tiles with particles are
+ * so few that all of them stay resident. */
 int icm_set_tile(icm_ctx *ctx, int tile_variant, int threads);
 int icm_get_tile(icm_ctx *ctx, int *tile_variant, int *threads);
 /* Fused forms: re-bin the particles by their current grid cell every
